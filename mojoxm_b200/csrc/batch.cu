@@ -42,7 +42,6 @@ struct BatchGroup {
   bool tc = false;
   int P = 0, kind = 0;
   Stage3DArgs<float>* d_margs = nullptr;  // [3][members]: stage arguments
-  KuhnTab3<float>* d_tabs = nullptr;      // [members]
   std::vector<int> members;  // indices into Batch::members
   int ec[6] = {0, 0, 0, 0, 0, 0};
   int4* d_items = nullptr;
@@ -195,11 +194,9 @@ void free_group(BatchGroup& g) {
   cudaFree(g.d_litems);
   cudaFree(g.d_counter);
   cudaFree(g.d_margs);
-  cudaFree(g.d_tabs);
   g.d_items = g.d_litems = nullptr;
   g.d_counter = nullptr;
   g.d_margs = nullptr;
-  g.d_tabs = nullptr;
 }
 
 // During the capture of the step the 3D members' single-solve launches go to
@@ -264,13 +261,11 @@ void build_tc3(Batch* b, BatchGroup& g) {
   if (ec < 1) throw ArgError("no tensor-core tile for this order and component count");
   std::vector<int4> items;
   std::vector<Stage3DArgs<float>> margs(size_t(3) * ng);
-  std::vector<KuhnTab3<float>> tabs(ng);
   for (int j = 0; j < ng; ++j) {
     Handle* h = b->members[g.members[j]];
     for (int64_t c0 = h->cbeg; c0 < h->cend; c0 += ec)
       items.push_back(make_int4(j, int(c0), int(std::min<int64_t>(ec, h->cend - c0)), 0));
     for (int st = 0; st < 3; ++st) margs[size_t(st) * ng + j] = tc_stage_args(h, st, b->dt[g.members[j]], b->derr);
-    tabs[j] = h->t3f;
   }
   order_tc3_items(h0, items);
   g.ec[g.P] = ec;
@@ -279,8 +274,6 @@ void build_tc3(Batch* b, BatchGroup& g) {
   CK(cudaMemcpy(g.d_items, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice));
   CK(cudaMalloc(&g.d_margs, margs.size() * sizeof(Stage3DArgs<float>)));
   CK(cudaMemcpy(g.d_margs, margs.data(), margs.size() * sizeof(Stage3DArgs<float>), cudaMemcpyHostToDevice));
-  CK(cudaMalloc(&g.d_tabs, tabs.size() * sizeof(KuhnTab3<float>)));
-  CK(cudaMemcpy(g.d_tabs, tabs.data(), tabs.size() * sizeof(KuhnTab3<float>), cudaMemcpyHostToDevice));
 }
 
 template <class R>
@@ -482,7 +475,7 @@ void build(Batch* b) {
   // occupancy) before the capture: an empty batch launches nothing
   for (auto& g : b->groups)
     if (g.dim == 3 && g.tc) {
-      const Tc3Batch none{g.d_margs, g.d_tabs, g.d_items, 0};
+      const Tc3Batch none{g.d_margs, g.d_items, 0};
       CK(launch_tc_group(b->members[g.members[0]], none, b->stream));
     }
   // side streams for the groups of a stage (a group's launch underfills the
@@ -518,7 +511,7 @@ void build(Batch* b) {
       if (g.dim == 2) {
         cap = launch_group_stage<R>(b, g, g.d_items, g.nitems, s, g.grid, g.smem, st);
       } else if (g.tc) {
-        const Tc3Batch bat{g.d_margs + size_t(s) * g.members.size(), g.d_tabs, g.d_items, g.nitems};
+        const Tc3Batch bat{g.d_margs + size_t(s) * g.members.size(), g.d_items, g.nitems};
         cap = launch_tc_group(b->members[g.members[0]], bat, st);
       } else {  // single-solve launches on the batch stream
         try {

@@ -58,18 +58,17 @@ static float bits_f32(uint32_t u) {
 }
 
 // Shared operator A (NP x K, row-major, FP64) as the tensor-core B operand:
-// N = NP rounded up to 16 rows; the volume columns [0, nvol) padded to
-// kvol = nvol rounded up to the MMA K step (16 for split-BF16, 8 for
+// a = hi + lo (bfloat16, or TF32 in 32-bit words), the NP rows of hi padded
+// to a multiple of 8, then those of lo; the volume columns [0, nvol) padded
+// to kvol = nvol rounded up to the MMA K step (16 for split-BF16, 8 for
 // split-TF32), then the face columns [nvol, K) from column kvol on, padded
-// likewise; K-major no-swizzle core-matrix layout, split into a hi image
-// followed by a lo image (a = hi + lo, bfloat16 or TF32 in 32-bit words);
-// padding entries are zero.
+// likewise; K-major no-swizzle core-matrix layout.  Padding rows and columns
+// are zeros.
 static std::vector<unsigned char> tc_operator_image(const std::vector<double>& A, int NP, int K, int nvol, int kind) {
   const int ks = kind == TC_TF32 ? 8 : 16, elem = kind == TC_TF32 ? 4 : 2;
-  const int NN = (NP + 15) / 16 * 16, kvol = (nvol + ks - 1) / ks * ks;
+  const int NR = (NP + 7) / 8 * 8, NN = 2 * NR, kvol = (nvol + ks - 1) / ks * ks;
   const int KA = kvol + (K - nvol + ks - 1) / ks * ks;
-  const size_t half = size_t(NN) * KA * elem;
-  std::vector<unsigned char> img(2 * half, 0);
+  std::vector<unsigned char> img(size_t(NN) * KA * elem, 0);
   for (int i = 0; i < NP; ++i)
     for (int k = 0; k < K; ++k) {
       const double v = A[size_t(i) * K + k];
@@ -77,15 +76,13 @@ static std::vector<unsigned char> tc_operator_image(const std::vector<double>& A
       if (kind == TC_TF32) {
         const uint32_t hi = tf32_bits(float(v));
         const uint32_t lo = tf32_bits(float(v - double(bits_f32(hi))));
-        const size_t off = umma_k_off<OpTF32>(i, col, NN);
-        std::memcpy(&img[off], &hi, 4);
-        std::memcpy(&img[half + off], &lo, 4);
+        std::memcpy(&img[umma_k_off<OpTF32>(i, col, NN)], &hi, 4);
+        std::memcpy(&img[umma_k_off<OpTF32>(NR + i, col, NN)], &lo, 4);
       } else {
         const uint16_t hi = bf16_bits(float(v));
         const uint16_t lo = bf16_bits(float(v - double(bf16_value(hi))));
-        const size_t off = umma_k_off<OpBF16>(i, col, NN);
-        std::memcpy(&img[off], &hi, 2);
-        std::memcpy(&img[half + off], &lo, 2);
+        std::memcpy(&img[umma_k_off<OpBF16>(i, col, NN)], &hi, 2);
+        std::memcpy(&img[umma_k_off<OpBF16>(NR + i, col, NN)], &lo, 2);
       }
     }
   return img;
@@ -137,12 +134,16 @@ void fill_tab3(Handle* h, KuhnTab3<R>& t) {
         t.nb_m[a][lf][m] = uint8_t(mm);
       }
     }
-  // work list of faces a cube evaluates once; a cube-boundary face must lead
-  // to the adjacent cube along its axis (the kernels resolve it per cube)
+  // work list of faces a cube evaluates once, the cube-boundary faces first
+  // (so that the threads of a warp mostly take faces of one sort); a
+  // cube-boundary face must lead to the adjacent cube along its axis (the
+  // kernels resolve it per cube)
   t.n_face_work = 0;
+  for (int inner = 0; inner < 2; ++inner)
   for (int a = 0; a < 6; ++a)
     for (int lf = 0; lf < 4; ++lf) {
       const int ax = k.axis[a][lf];
+      if ((ax < 0) != (inner == 1)) continue;
       if (ax >= 0) {
         for (int d = 0; d < 3; ++d)
           if (k.off[a][lf][d] != (d == ax ? k.dir[a][lf] : 0)) throw ArgError("internal: cube face offset");
@@ -151,8 +152,33 @@ void fill_tab3(Handle* h, KuhnTab3<R>& t) {
           if (k.off[a][lf][d] != 0) throw ArgError("internal: inner face offset");
         if (k.side[a][lf] != 0) continue;
       }
+      if (t.n_face_work == kFaceWork3 || (ax >= 0) != (t.n_face_work < kCubeFaces3))
+        throw ArgError("internal: Kuhn face work list");
       t.face_work[t.n_face_work++] = uint8_t(a * 4 + lf);
     }
+}
+
+// The tensor-core stage's form of a solve's topology table.
+static Tc3Tab tc3_table(const Handle* h) {
+  const KuhnTab3<float>& k = h->t3f;
+  Tc3Tab t;
+  std::memset(&t, 0, sizeof(t));
+  for (int a = 0; a < 6; ++a)
+    for (int r = 0; r < 7; ++r)
+      for (int d = 0; d < 3; ++d)
+        t.dir[a][r][d][0] = t.dir[a][r][d][1] = r < 3 ? k.invJ[a][r * 3 + d] : k.normal[a][r - 3][d];
+  for (int w = 0; w < kFaceWork3; ++w) {
+    const int a = k.face_work[w] >> 2, lf = k.face_work[w] & 3, ax = k.axis[a][lf], nbt = k.nb_t[a][lf],
+              lf2 = k.nb_lf[a][lf];
+    Tc3Tab::Face& f = t.face[w];
+    f.scale[0] = f.scale[1] = 0.5f * k.fscale[a][lf];
+    f.scale2[0] = f.scale2[1] = ax < 0 ? 0.5f * k.fscale[nbt][lf2] : 0.0f;
+    f.bits = a | (lf << 3) | ((nbt & 7) << 5) | ((lf2 & 3) << 8) |
+             (ax >= 0 ? (2 * ax + (k.dir[a][lf] > 0 ? 1 : 0)) << 12 : 0) | ((k.side[a][lf] == 0 ? 1 : 0) << 15);
+    for (int m = 0; m < h->NFP; ++m)
+      t.nodes[w * h->NFP + m] = int(k.own_node[lf][m]) | (int(k.nb_node[a][lf][m]) << 8) | (int(k.nb_m[a][lf][m]) << 16);
+  }
+  return t;
 }
 
 template <class R>
@@ -270,6 +296,7 @@ Stage3DArgs<R> stage3d_args(const Handle* h, const void* qi, const void* qa, con
   for (int k = 0; k < 6; ++k) ar.bc[k] = h->bc[k];
   ar.rhs_only = rhs_only;
   ar.err = h->derr;
+  ar.tctab = h->use_tc ? (const Tc3Tab*)((const unsigned char*)h->tcimg + h->tctab_off) : nullptr;
   return ar;
 }
 
@@ -312,7 +339,7 @@ cudaError_t stage_launch(Handle* h, const void* qi, const void* qa, const void* 
     return with_phys3d<R>(h, [&](const auto& ph) -> cudaError_t {
       if constexpr (std::is_same<R, float>::value && std::decay<decltype(ph)>::type::NC <= 16) {
         if (h->use_tc)
-          return launch_stage3d_tc(h->P, h->tc_kind, ar, t, ph, (const unsigned char*)h->tcimg, h->nsm, h->stream);
+          return launch_stage3d_tc(h->P, h->tc_kind, ar, ph, (const unsigned char*)h->tcimg, h->nsm, h->stream);
       }
       return launch_stage3d<R>(h->P, ar, t, ph, h->nsm, h->stream);
     });
@@ -863,6 +890,10 @@ Handle* create(const mxm_dg_mesh_desc* m, const mxm_dg_physics_desc* ph, int P, 
     upload(&raw->w, raw->ref.w);
     if (raw->use_tc) {
       auto img = tc_operator_image(raw->Ahost, raw->NP, raw->K, 3 * raw->NP, raw->tc_kind);
+      raw->tctab_off = (img.size() + 15) / 16 * 16;
+      img.resize(raw->tctab_off + sizeof(Tc3Tab));
+      const Tc3Tab t = tc3_table(raw);
+      std::memcpy(&img[raw->tctab_off], &t, sizeof(t));
       dev_alloc(raw, &raw->tcimg, img.size());
       CK(cudaMemcpyAsync(raw->tcimg, img.data(), img.size(), cudaMemcpyHostToDevice, raw->stream));
       CK(cudaStreamSynchronize(raw->stream));  // img goes out of scope

@@ -35,6 +35,27 @@ struct KuhnTab3 {
   int32_t n_face_work;
 };
 
+// The same topology as the tensor-core stage reads it, decoded once per solve
+// on the host (device memory beside the operator image; tc3tab_bytes(P) of
+// it): directions and scales duplicated into lane pairs for packed FP32
+// arithmetic, faces in work-list order.
+// The work list of a Kuhn cube has 12 cube faces, then 6 faces inside the cube.
+constexpr int kCubeFaces3 = 12, kFaceWork3 = 18;
+struct Tc3Tab {
+  float dir[6][7][3][2];  // per tet type: the invJ rows, then the face normals (side 0 -> side 1)
+  struct Face {
+    float scale[2];   // fscale / 2 of the face
+    float scale2[2];  // ... of the same face seen from the other tet (faces inside a cube)
+    // t | lf << 3 | nb_t << 5 | nb_lf << 8 | (2 axis + (dir > 0)) << 12 (cube faces) | (side == 0) << 15
+    int bits, pad;
+  } face[kFaceWork3];
+  int nodes[kFaceWork3 * kMaxNFP3];  // [work][NFP]: own node | neighbour's node << 8 | neighbour's face index << 16
+  int pad[2];
+};
+__host__ __device__ constexpr size_t tc3tab_bytes(int P) {
+  return (sizeof(Tc3Tab) - sizeof(int) * (kFaceWork3 * (kMaxNFP3 - ntri(P)) + 2) + 15) / 16 * 16;
+}
+
 template <class R>
 struct KuhnTab2 {
   R normal[2][3][2];
@@ -109,20 +130,29 @@ __device__ __forceinline__ int face_mode(int axis, int dir, int cpos, int ncell_
 
 __device__ __forceinline__ int wrapi(int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); }
 
-// Neighbour cube and face treatment of the six cube faces of one cube,
+// a / b of a cell count (0 <= a < 2^24, b >= 1) through the FP32 reciprocal:
+// the rounded quotient is at most one off, which the remainder corrects
+// (an integer division costs several times the instructions).
+__device__ __forceinline__ int div_cells(int a, int b) {
+  int k = int(__fdividef(float(a), float(b)));
+  const int r = a - k * b;
+  k += (r >= b) - (r < 0);
+  return k;
+}
+
+// Neighbour cube and face treatment of one of the six cube faces of a cube,
 // resolved once per tile so the face-node loops do no integer division.
-// Direction index dd = 2 * axis + (dir > 0).  nb[dd] = neighbour cube
-// (periodic wrap), md[dd] = face mode | BC code << 8.
-__device__ __forceinline__ void cube_dirs3(int cell, int nx, int ny, int nz, const int* bc, int* nb, int* md, int dd) {
+// Direction index dd = 2 * axis + (dir > 0); returns {neighbour cube
+// (periodic wrap), face mode | BC code << 8}.
+__device__ __forceinline__ int2 cube_dir3(int cell, int nx, int ny, int nz, const int* bc, int dd) {
   const int nxy = nx * ny;
-  const int ck = cell / nxy, rem = cell - ck * nxy, cj = rem / nx, ci = rem - cj * nx;
+  const int ck = div_cells(cell, nxy), rem = cell - ck * nxy, cj = div_cells(rem, nx), ci = rem - cj * nx;
   const int ax = dd >> 1, dir = (dd & 1) ? 1 : -1;
   int code;
   const int mode = face_mode(ax, dir, ax == 0 ? ci : (ax == 1 ? cj : ck), ax == 0 ? nx : (ax == 1 ? ny : nz), bc, code);
   const int ni = ax == 0 ? wrapi(ci + dir, nx) : ci, nj = ax == 1 ? wrapi(cj + dir, ny) : cj,
             nk = ax == 2 ? wrapi(ck + dir, nz) : ck;
-  nb[dd] = ni + nx * (nj + ny * nk);
-  md[dd] = mode | (code << 8);
+  return make_int2(ni + nx * (nj + ny * nk), mode | (code << 8));
 }
 
 // Resident blocks per SM of a persistent kernel with `nt` threads and `smem`
@@ -191,6 +221,7 @@ struct Stage3DArgs {
   int bc[6];
   int rhs_only;
   int* err;  // device error word (bounded waits that gave up set bit 0)
+  const Tc3Tab* tctab;  // tensor-core stage: its topology table (null otherwise)
 };
 
 template <class R>
@@ -235,10 +266,9 @@ cudaError_t launch_wavespeed3d(int P, const Stage3DArgs<R>& a, const KuhnTab3<R>
 // order and operand kind in one launch.  items[t] = {solve, first cell,
 // cells, 0}, the tiles of one solve consecutive; margs[solve] are the
 // solve's arguments of the stage launched (q_in / q_a / q_b / q_out, b,
-// c dt, mesh, boundaries), tabs[solve] its metric table.
+// c dt, mesh, boundaries, topology table).
 struct Tc3Batch {
   const Stage3DArgs<float>* margs;
-  const KuhnTab3<float>* tabs;
   const int4* items;
   int nitems;
 };
@@ -254,8 +284,8 @@ cudaError_t stage3d_tc_batch_grid(int P, int kind, const Phys& ph, int nsm, int 
 // `img` is the operator image built by tc_operator_image() for that kind.
 constexpr int TC_BF16 = 0, TC_TF32 = 1;
 template <class Phys>
-cudaError_t launch_stage3d_tc(int P, int kind, const Stage3DArgs<float>& a, const KuhnTab3<float>& tab,
-                              const Phys& ph, const unsigned char* img, int nsm, cudaStream_t st);
+cudaError_t launch_stage3d_tc(int P, int kind, const Stage3DArgs<float>& a, const Phys& ph, const unsigned char* img,
+                              int nsm, cudaStream_t st);
 // Whether the tensor-core stage of (P, components, kind) fits one block's
 // shared memory.
 bool tc_shape_fits(int P, int NC, int kind);

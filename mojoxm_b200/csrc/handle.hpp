@@ -71,7 +71,8 @@ struct Handle {
   int* derr = nullptr;  // device error word written by bounded waits
   bool use_tc = false;  // MIXED / MIXED_TF32 precision: tensor-core contraction
   int tc_kind = 0;      // TC_BF16 or TC_TF32 operands
-  void* tcimg = nullptr;  // operator image (bf16 hi | lo) in the UMMA layout
+  void* tcimg = nullptr;  // operator image (bf16 hi | lo) in the UMMA layout, then the Tc3Tab at tctab_off
+  size_t tctab_off = 0;
   int npartial = 1024;
   bool lim_on = false;
   double lim_eps = 0.1;

@@ -1,0 +1,300 @@
+// Packed-FP32 forms of the 3D physics: the tensor-core stage evaluates its
+// fluxes for the same node of two neighbouring cubes at once, so every index,
+// metric term and normal is shared by the two lanes and the instruction count
+// of the arithmetic halves.
+#pragma once
+#include "f32x2.cuh"
+#include "physics.cuh"
+
+namespace mxm {
+
+// fmaxf returns the other operand for a NaN, as `x > floor ? x : floor` does
+__device__ __forceinline__ f2 max2(f2 x, float lo) { return each2(x, [lo](float a) { return fmaxf(a, lo); }); }
+__device__ __forceinline__ f2 max2(f2 x, f2 y) { return each2(x, y, [](float a, float b) { return fmaxf(a, b); }); }
+__device__ __forceinline__ f2 min2(f2 x, f2 y) { return each2(x, y, [](float a, float b) { return fminf(a, b); }); }
+__device__ __forceinline__ f2 abs2(f2 x) { return each2(x, [](float a) { return fabsf(a); }); }
+__device__ __forceinline__ f2 absadd2(f2 x, f2 y) { return each2(x, y, [](float a, float b) { return fabsf(a) + b; }); }
+__device__ __forceinline__ f2 rcp2(f2 x) { return each2(x, [](float a) { return pos_rcp(a); }); }
+// hardware square root (0 -> 0), as accurate as the reciprocal square root
+// that pos_sqrt uses
+__device__ __forceinline__ float sqrt_hw(float x) {
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ f2 sqrt2(f2 x) { return each2(x, [](float a) { return sqrt_hw(a); }); }
+// quotient, divisor of either sign
+__device__ __forceinline__ f2 div2(f2 x, f2 y) {
+  return each2(x, y, [](float a, float b) { return __fdividef(a, b); });
+}
+__device__ __forceinline__ f2 dot2(const f2* a, f2 x, f2 y, f2 z) { return fma2(a[2], z, fma2(a[1], y, a[0] * x)); }
+
+// The pair form of a 3D physics (float): flux() is the physical flux F[d * NC
+// + c]; face() is TWICE the numerical flux of (l, r) along the unit normal n
+// (every flux here is a half sum, so the factor goes into the face scale)
+// less `b`, twice the element's constant normal flux: taken off early in each
+// sum, so that the sum's later roundings are those of the flux variation and
+// not of the flux.  The formulas are those of physics.cuh.
+template <class Phys>
+struct PairPhys;
+
+template <>
+struct PairPhys<AdvectionD<float>> {
+  using Ph = AdvectionD<float>;
+  __device__ __forceinline__ static void flux(const Ph& ph, const f2* q, f2* F) {
+    F[0] = dup2(ph.vx) * q[0];
+    F[1] = dup2(ph.vy) * q[0];
+    F[2] = dup2(ph.vz) * q[0];
+  }
+  __device__ __forceinline__ static void face(const Ph& ph, const f2* l, const f2* r, const f2* n, const f2* b, f2* f) {
+    const f2 nc = fma2(dup2(ph.vz), n[2], fma2(dup2(ph.vy), n[1], dup2(ph.vx) * n[0])), a = abs2(nc);
+    f[0] = fma2(nc + a, l[0], fma2(nc - a, r[0], b[0] * dup2(-1.0f)));
+  }
+};
+
+template <int FLUX>
+struct PairPhys<EulerD<float, FLUX>> {
+  using Ph = EulerD<float, FLUX>;
+  struct Pre {
+    f2 ri, p;
+  };
+  __device__ __forceinline__ static void pre(const Ph& ph, const f2* q, Pre& a) {
+    a.ri = rcp2(max2(q[0], ph.rho_min));
+    const f2 mm = fma2(q[3], q[3], fma2(q[2], q[2], q[1] * q[1]));
+    a.p = max2(fma2(mm, a.ri * dup2(-0.5f), q[4]) * dup2(ph.gamma - 1.0f), ph.p_min);
+  }
+  __device__ __forceinline__ static void flux(const Ph& ph, const f2* q, f2* F) {
+    Pre a;
+    pre(ph, q, a);
+    const f2 u = q[1] * a.ri, v = q[2] * a.ri, w = q[3] * a.ri, H = q[4] + a.p;
+    F[0] = q[1], F[5] = q[2], F[10] = q[3];
+    F[1] = fma2(q[1], u, a.p), F[7] = fma2(q[2], v, a.p), F[13] = fma2(q[3], w, a.p);
+    F[2] = F[6] = q[1] * v, F[3] = F[11] = q[1] * w, F[8] = F[12] = q[2] * w;
+    F[4] = u * H, F[9] = v * H, F[14] = w * H;
+  }
+  __device__ __forceinline__ static void face(const Ph& ph, const f2* l, const f2* r, const f2* n, const f2* b, f2* f) {
+    if constexpr (FLUX == FLUX_RUSANOV) {
+      Pre x, y;
+      pre(ph, l, x);
+      pre(ph, r, y);
+      const f2 ga = dup2(ph.gamma);
+      const f2 mnl = dot2(l + 1, n[0], n[1], n[2]), mnr = dot2(r + 1, n[0], n[1], n[2]);
+      const f2 ul = mnl * x.ri, ur = mnr * y.ri;
+      const f2 c = max2(absadd2(ul, sqrt2(ga * x.p * x.ri)), absadd2(ur, sqrt2(ga * y.p * y.ri)));
+      const f2 ps = x.p + y.p;
+      // (floored densities in the dissipation, as in the scalar form)
+      f[0] = fma2(c, max2(l[0], ph.rho_min) - max2(r[0], ph.rho_min), (mnl - b[0]) + mnr);
+#pragma unroll
+      for (int k = 1; k < 4; ++k)
+        f[k] = fma2(l[k], ul, fma2(r[k], ur, fma2(c, l[k] - r[k], fma2(ps, n[k - 1], b[k] * dup2(-1.0f)))));
+      f[4] = fma2(l[4] + x.p, ul, fma2(r[4] + y.p, ur, c * (l[4] - r[4]) - b[4]));
+    } else if constexpr (FLUX == FLUX_HLLE || FLUX == FLUX_HLLEC) {
+      if (ph.entropy_fix) return lanes(ph, l, r, n, b, f);
+      // fluxes, Roe-averaged signal speeds (euler.mojo:161-176, :364-485) in
+      // the world frame: the face-frame rotation pair drops out
+      Pre x, y;
+      pre(ph, l, x);
+      pre(ph, r, y);
+      const f2 ga = dup2(ph.gamma), rl = max2(l[0], ph.rho_min), rr = max2(r[0], ph.rho_min);
+      const f2 mnl = dot2(l + 1, n[0], n[1], n[2]), mnr = dot2(r + 1, n[0], n[1], n[2]);
+      const f2 ul = mnl * x.ri, ur = mnr * y.ri;
+      f2 s0, s2;
+      {
+        const f2 il = sqrt2(x.ri), ir = sqrt2(y.ri), is = rcp2(fma2(rl, il, rr * ir));  // sqrt(rho) = rho / sqrt(rho)
+        const f2 wl = il * is, wr = ir * is;
+        const f2 vx = fma2(l[1], wl, r[1] * wr), vy = fma2(l[2], wl, r[2] * wr), vz = fma2(l[3], wl, r[3] * wr);
+        const f2 H = fma2(l[4] + x.p, wl, (r[4] + y.p) * wr);
+        const f2 v2 = fma2(vz, vz, fma2(vy, vy, vx * vx));
+        const f2 c = sqrt2(max2((H - dup2(0.5f) * v2) * dup2(ph.gamma - 1.0f), 0.0f));
+        const f2 u = fma2(vz, n[2], fma2(vy, n[1], vx * n[0]));
+        s0 = min2(ul - sqrt2(ga * x.p * x.ri), u - c);
+        s2 = max2(ur + sqrt2(ga * y.p * y.ri), u + c);
+      }
+      // Both solvers' dissipation sum_k |s_k| W_k in terms of the jump r - l
+      // (and fr - fl, or the star states' distance from their own side): every
+      // factor is a difference already, so nothing of the states' size cancels
+      // and the waves themselves are never formed.
+      const f2 a0 = abs2(s0), a2 = abs2(s2);
+      if constexpr (FLUX == FLUX_HLLE) {
+        // W0 = (s2 dq - df) / (s2 - s0), W2 = (df - s0 dq) / (s2 - s0)
+        const f2 iden = rcp2(s2 - s0), al = (a2 - a0) * iden, be = (a0 * s2 - a2 * s0) * iden;
+        auto comp = [&](int k, f2 fl, f2 fr) {
+          f[k] = (fl - b[k]) + fr - fma2(al, fr - fl, be * (r[k] - l[k]));
+        };
+        comp(0, mnl, mnr);
+#pragma unroll
+        for (int k = 1; k < 4; ++k) comp(k, fma2(l[k], ul, x.p * n[k - 1]), fma2(r[k], ur, y.p * n[k - 1]));
+        comp(4, (l[4] + x.p) * ul, (r[4] + y.p) * ur);
+      } else {
+        // star state less its own side: q e + rho (1 + e) (s1 - un) (0, n, s1 + p / (rho (s - un))),
+        // e = (s1 - un) / (s - s1)
+        const f2 ml = rl * (s0 - ul), mr = rr * (s2 - ur);
+        const f2 s1 = div2((y.p - x.p) + (ul * ml - ur * mr), ml - mr), a1 = abs2(s1);
+        const f2 tl = s1 - ul, tr = s1 - ur, el = div2(tl, s0 - s1), er = div2(tr, s2 - s1);
+        const f2 kl = fma2(rl, el, rl) * tl, kr = fma2(rr, er, rr) * tr;
+        const f2 w0 = a0 - a1, w2 = a1 - a2, ps = x.p + y.p;
+        // s: fl + fr - b; dl, dr: the star states less their own side
+        auto comp = [&](int k, f2 s, f2 dl, f2 dr) {
+          f[k] = s - fma2(w0, dl, fma2(w2, dr, a1 * (r[k] - l[k])));
+        };
+        comp(0, (mnl - b[0]) + mnr, fma2(rl, el, rl - l[0]), fma2(rr, er, rr - r[0]));
+#pragma unroll
+        for (int k = 1; k < 4; ++k)
+          comp(k, fma2(l[k], ul, fma2(r[k], ur, fma2(ps, n[k - 1], b[k] * dup2(-1.0f)))),
+               fma2(l[k], el, kl * n[k - 1]), fma2(r[k], er, kr * n[k - 1]));
+        comp(4, fma2(l[4] + x.p, ul, (r[4] + y.p) * ur - b[4]), fma2(l[4], el, kl * (s1 + div2(x.p, ml))),
+             fma2(r[4], er, kr * (s1 + div2(y.p, mr))));
+      }
+    } else {
+      lanes(ph, l, r, n, b, f);
+    }
+  }
+  // the scalar solver once per lane (Roe, and the Harten-Hyman fix)
+  __device__ static void lanes(const Ph& ph, const f2* l, const f2* r, const f2* n, const f2* b, f2* f) {
+    float lx[2][5], rx[2][5], nx[2][3], fx[2][5];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+      un2(l[c], lx[0][c], lx[1][c]);
+      un2(r[c], rx[0][c], rx[1][c]);
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) un2(n[d], nx[0][d], nx[1][d]);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) ph.num_flux(lx[k], rx[k], nx[k][0], nx[k][1], nx[k][2], fx[k]);
+#pragma unroll
+    for (int c = 0; c < 5; ++c) f[c] = mk2(2.0f * fx[0][c], 2.0f * fx[1][c]) - b[c];
+  }
+};
+
+template <>
+struct PairPhys<MaxwellD<float>> {
+  using Ph = MaxwellD<float>;
+  __device__ __forceinline__ static void flux(const Ph& ph, const f2* q, f2* F) {
+    const f2 c2 = dup2(ph.c * ph.c), z = dup2(0.0f), bx = c2 * q[3], by = c2 * q[4], bz = c2 * q[5];
+    F[0] = z, F[1] = bz, F[2] = z - by, F[3] = z, F[4] = z - q[2], F[5] = q[1];
+    F[6] = z - bz, F[7] = z, F[8] = bx, F[9] = q[2], F[10] = z, F[11] = z - q[0];
+    F[12] = by, F[13] = z - bx, F[14] = z, F[15] = z - q[1], F[16] = q[0], F[17] = z;
+  }
+  // flux along g: (-c^2 g x B, g x E)
+  __device__ __forceinline__ static void normal(const Ph& ph, const f2* q, const f2* g, f2* F) {
+    const f2 c2 = dup2(ph.c * ph.c);
+    F[0] = c2 * (q[4] * g[2] - q[5] * g[1]);
+    F[1] = c2 * (q[5] * g[0] - q[3] * g[2]);
+    F[2] = c2 * (q[3] * g[1] - q[4] * g[0]);
+    F[3] = q[2] * g[1] - q[1] * g[2];
+    F[4] = q[0] * g[2] - q[2] * g[0];
+    F[5] = q[1] * g[0] - q[0] * g[1];
+  }
+  // linear: the flux of the sum of the two states, and the jump
+  __device__ __forceinline__ static void face(const Ph& ph, const f2* l, const f2* r, const f2* n, const f2* b, f2* f) {
+    f2 s[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) s[k] = l[k] + r[k];
+    normal(ph, s, n, f);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) f[k] = fma2(dup2(ph.c), l[k] - r[k], f[k] - b[k]);
+  }
+};
+
+template <>
+struct PairPhys<ShallowWaterD<float>> {
+  using Ph = ShallowWaterD<float>;
+  struct Pre {
+    f2 h, ri, p;
+  };
+  __device__ __forceinline__ static void pre(const Ph& ph, const f2* q, Pre& a) {
+    a.h = max2(q[0], ph.h_min);
+    a.ri = rcp2(a.h);
+    a.p = dup2(0.5f * ph.g) * a.h * a.h;
+  }
+  __device__ __forceinline__ static void flux(const Ph& ph, const f2* q, f2* F) {
+    Pre a;
+    pre(ph, q, a);
+    const f2 u = q[1] * a.ri, v = q[2] * a.ri, z = dup2(0.0f);
+    F[0] = q[1], F[1] = fma2(q[1], u, a.p), F[2] = q[1] * v;
+    F[3] = q[2], F[4] = F[2], F[5] = fma2(q[2], v, a.p);
+    F[6] = F[7] = F[8] = z;
+  }
+  __device__ __forceinline__ static void normal(const Ph&, const f2* q, const Pre& a, const f2* g, f2* F) {
+    F[0] = fma2(q[2], g[1], q[1] * g[0]);
+    const f2 un = F[0] * a.ri;
+    F[1] = fma2(q[1], un, a.p * g[0]);
+    F[2] = fma2(q[2], un, a.p * g[1]);
+  }
+  __device__ __forceinline__ static void face(const Ph& ph, const f2* l, const f2* r, const f2* n, const f2* b, f2* f) {
+    Pre x, y;
+    pre(ph, l, x);
+    pre(ph, r, y);
+    f2 fl[3], fr[3];
+    normal(ph, l, x, n, fl);
+    normal(ph, r, y, n, fr);
+    const f2 al = max2(absadd2(fl[0] * x.ri, sqrt2(dup2(ph.g) * x.h)), absadd2(fr[0] * y.ri, sqrt2(dup2(ph.g) * y.h)));
+#pragma unroll
+    for (int k = 0; k < 3; ++k) f[k] = fma2(al, l[k] - r[k], (fl[k] - b[k]) + fr[k]);
+  }
+};
+
+template <>
+struct PairPhys<MhdD<float>> {
+  using Ph = MhdD<float>;
+  struct Pre {
+    f2 ri, p, b2, pt, ub;  // 1/rho, gas pressure, |B|^2, total pressure, u.B
+  };
+  __device__ __forceinline__ static void pre(const Ph& ph, const f2* q, Pre& a) {
+    const f2 h = dup2(0.5f);
+    a.ri = rcp2(max2(q[0], ph.rho_min));
+    const f2 ke = fma2(q[3], q[3], fma2(q[2], q[2], q[1] * q[1])) * (a.ri * h);
+    a.b2 = fma2(q[7], q[7], fma2(q[6], q[6], q[5] * q[5]));
+    a.p = max2((q[4] - ke - a.b2 * h) * dup2(ph.gamma - 1.0f), ph.p_min);
+    a.pt = fma2(a.b2, h, a.p);
+    a.ub = fma2(q[3], q[7], fma2(q[2], q[6], q[1] * q[5])) * a.ri;
+  }
+  __device__ __forceinline__ static void flux(const Ph& ph, const f2* q, f2* F) {
+    Pre a;
+    pre(ph, q, a);
+    const f2 u = q[1] * a.ri, v = q[2] * a.ri, w = q[3] * a.ri, H = q[4] + a.pt, ch2 = dup2(ph.c_h * ph.c_h);
+    F[0] = q[1], F[9] = q[2], F[18] = q[3];
+    F[1] = fma2(q[1], u, a.pt) - q[5] * q[5];
+    F[11] = fma2(q[2], v, a.pt) - q[6] * q[6];
+    F[21] = fma2(q[3], w, a.pt) - q[7] * q[7];
+    F[2] = F[10] = q[1] * v - q[5] * q[6];
+    F[3] = F[19] = q[1] * w - q[5] * q[7];
+    F[12] = F[20] = q[2] * w - q[6] * q[7];
+    F[4] = u * H - q[5] * a.ub, F[13] = v * H - q[6] * a.ub, F[22] = w * H - q[7] * a.ub;
+    F[5] = F[15] = F[25] = q[8];
+    F[6] = u * q[6] - v * q[5], F[14] = v * q[5] - u * q[6];
+    F[7] = u * q[7] - w * q[5], F[23] = w * q[5] - u * q[7];
+    F[16] = v * q[7] - w * q[6], F[24] = w * q[6] - v * q[7];
+    F[8] = ch2 * q[5], F[17] = ch2 * q[6], F[26] = ch2 * q[7];
+  }
+  // flux along n
+  __device__ __forceinline__ static void normal(const Ph& ph, const f2* q, const Pre& a, const f2* g, f2* F) {
+    const f2 mg = dot2(q + 1, g[0], g[1], g[2]), bg = dot2(q + 5, g[0], g[1], g[2]), un = mg * a.ri, w = bg * a.ri;
+    F[0] = mg;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      F[1 + k] = fma2(q[1 + k], un, a.pt * g[k]) - q[5 + k] * bg;
+      F[5 + k] = fma2(q[5 + k], un, q[8] * g[k]) - q[1 + k] * w;
+    }
+    F[4] = un * (q[4] + a.pt) - bg * a.ub;
+    F[8] = dup2(ph.c_h * ph.c_h) * bg;
+  }
+  __device__ __forceinline__ static f2 fast(const Ph& ph, const f2* q, const Pre& a, const f2* n) {
+    const f2 bn = dot2(q + 5, n[0], n[1], n[2]), cs2 = dup2(ph.gamma) * a.p * a.ri, ca2 = a.b2 * a.ri;
+    const f2 s = cs2 + ca2, disc = max2(s * s - dup2(4.0f) * cs2 * (bn * bn * a.ri), 0.0f);
+    return sqrt2(dup2(0.5f) * (s + sqrt2(disc)));
+  }
+  __device__ __forceinline__ static void face(const Ph& ph, const f2* l, const f2* r, const f2* n, const f2* b, f2* f) {
+    Pre x, y;
+    pre(ph, l, x);
+    pre(ph, r, y);
+    f2 g[9];
+    normal(ph, l, x, n, f);
+    normal(ph, r, y, n, g);
+    const f2 al = max2(max2(absadd2(f[0] * x.ri, fast(ph, l, x, n)), absadd2(g[0] * y.ri, fast(ph, r, y, n))), ph.c_h);
+#pragma unroll
+    for (int c = 0; c < 9; ++c) f[c] = fma2(al, l[c] - r[c], (f[c] - b[c]) + g[c]);
+  }
+};
+
+}  // namespace mxm

@@ -176,7 +176,9 @@ __global__ void __launch_bounds__(NT) stage3d_kernel(Stage3DArgs<R> args, KuhnTa
     }
     for (int w = tid; w < nhere * 6; w += NT) {
       const int cl = w / 6, dd = w - cl * 6;
-      cube_dirs3(cell0 + cl, args.nx, args.ny, args.nz, args.bc, sNb + cl * 6, sMd + cl * 6, dd);
+      const int2 cd = cube_dir3(cell0 + cl, args.nx, args.ny, args.nz, args.bc, dd);
+      sNb[w] = cd.x;
+      sMd[w] = cd.y;
     }
     __syncthreads();
     // ---- volume fluxes in reference coordinates -> B rows k*NP + j

@@ -1,16 +1,18 @@
 // Mixed-precision 3D stage kernel: FP32 state, fluxes and Riemann solves,
 // the volume + lift contraction on the 5th-generation tensor cores
-// (tcgen05.mma, split-BF16 operands, FP32 accumulation in tensor memory).
+// (tcgen05.mma, split-BF16 or split-TF32 operands, FP32 accumulation in
+// tensor memory).
 //
-// Same dataflow as stage3d_kernel (whole cubes per tile, bulk-copied
-// double-buffered state, implicit connectivity), with the contraction in
+// Same dataflow as stage3d_kernel (whole cubes per tile, bulk-copied state,
+// implicit connectivity), with the contraction in
 // the transposed form
-//     RHS^T[(c,el), i] = sum_k  B^T[(c,el), k] * A[i, k]
+//     RHS^T[(c,slot), i] = sum_k  B^T[(c,slot), k] * A[i, k]
 // so one 128-row MMA tile covers the (component, element) pairs of a tile
-// against the shared operator A (N = NP rounded up to 16, K = 3NP + 4NFP
+// against the shared operator A (N = 2 NP rounded up, K = 3NP + 4NFP
 // rounded up to the MMA K step).  Operands are split x = hi + lo in
-// bfloat16 (kind::f16) or TF32 (kind::tf32) and the product is
-// hi*hi + hi*lo + lo*hi (three MMAs into one FP32 accumulator).
+// bfloat16 (kind::f16) or TF32 (kind::tf32); flux hi and flux lo each meet
+// [operator hi | operator lo] in one MMA, and the two halves of the FP32
+// accumulator are added when they are read.
 //
 // Accuracy: before splitting, every element subtracts its own constant flux
 // Fbar = F(q at node 0) from its volume fluxes and Fbar.n from its face
@@ -20,26 +22,39 @@
 // cancellation error of the O(|F|/h) terms -- shrink to the flux variation
 // across the element.
 //
-// Layout: the (c,el) x K operand is MN-major for split-BF16 (8 consecutive
+// What binds it and the mapping that follows: the kernel is bound by its
+// instruction stream (fluxes, conversions and index arithmetic of 24 warps
+// per SM), far from the HBM and tensor rooflines, so the mapping is chosen
+// for the fewest instructions per value.
+//  * A thread evaluates the same node (or face node) of two neighbouring
+//    cubes of the tile in packed FP32 arithmetic (pair.cuh): the tet type,
+//    node numbers, metric rows, normals and scales are those of both.
+//  * Rows are ordered by tet type, then cube (slot = t * EC + cube), so the
+//    two values of a pair are neighbouring rows: in the MN-major split-BF16
+//    tile one packed conversion and one 4-byte store for each of hi and lo.
+//  * Metric rows, normals and face records arrive decoded and duplicated
+//    into lane pairs (Tc3Tab, built once per solve on the host).
+//
+// Layout: the (c,slot) x K operand is MN-major for split-BF16 (8 consecutive
 // rows of one k in 16 bytes) and K-major for split-TF32 (4 consecutive k of
-// one row in 16 bytes).  Work is mapped element-fastest: 8 consecutive threads take 8
-// consecutive elements at the same node, so a warp's operand stores land in
-// one or two 128-byte core matrices.  Faces are walked through a per-cube
-// work list (every cube-boundary face, and each face inside the cube once,
-// by its side-0 tet, which writes both tets' rows); the neighbour cube and
-// boundary treatment of the six cube faces are resolved once per tile.  One
-// thread issues the MMAs; completion is tracked by tcgen05.commit on an
-// mbarrier with a bounded wait; warps 0-3 read the accumulator with
-// tcgen05.ld into a padded [row][i] staging tile for the FP32 epilogue
-// (source, RK combine, positivity floor).
+// one row in 16 bytes).  Faces are walked through a per-cube work list
+// (every cube-boundary face, and each face inside the cube once, by its
+// side-0 tet, which writes both tets' rows); the neighbour cube and boundary
+// treatment of the six cube faces are resolved once per tile.  One thread
+// issues the MMAs; completion is tracked by tcgen05.commit on an mbarrier
+// with a bounded wait; the warps read the accumulator with tcgen05.ld into a
+// padded [row][i] staging tile for the FP32 epilogue (source, RK combine,
+// positivity floor).
 #pragma once
+#include <type_traits>
+
 #include "dg_common.cuh"
+#include "pair.cuh"
 #include "physics.cuh"
 #include "tc.cuh"
 
 namespace mxm {
 
-__host__ __device__ constexpr int rup16(int x) { return (x + 15) / 16 * 16; }
 __host__ __device__ constexpr int rupk(int x, int k) { return (x + k - 1) / k * k; }
 __host__ __device__ constexpr int tmem_cols_for(int n) { return n <= 32 ? 32 : (n <= 64 ? 64 : (n <= 128 ? 128 : 256)); }
 
@@ -48,121 +63,114 @@ __host__ __device__ constexpr int tmem_cols_for(int n) { return n <= 32 ? 32 : (
 // MMA K step; both halves reuse one operand buffer of KB = max(KV, KF)
 // columns, and the operator image stores the face columns from KV on
 // (tc_operator_image's `kvol`).
+//
+// Shared memory decides how many blocks an SM holds, so both operands keep
+// only the core matrices they need: the operator's hi rows are followed by
+// its lo rows (NR = NP rounded up to 8 each) in one N = 2 NR operand, and the
+// flux tile has RB = its used rows rounded up to 8.  The MMA still covers
+// M = 128 rows: core matrices past RB are read from whatever follows in
+// shared memory, and feed accumulator rows that nobody reads.
 template <int P, int NC, class Op = OpBF16>
 struct TcShape {
   static constexpr int NP = ntet(P), NFP = ntri(P), K = 3 * NP + 4 * NFP;
   static constexpr int KV = rupk(3 * NP, Op::KSTEP), KF = rupk(4 * NFP, Op::KSTEP), KA = KV + KF;
   static constexpr int KB = KV > KF ? KV : KF;
-  static constexpr int NN = rup16(NP), M = 128;
-  static constexpr int EBP = (M / NC) / 8 * 8;      // element slots per component (multiple of 8)
-  static constexpr int EC = EBP / 6, EB = 6 * EC;   // whole cubes in a tile
-  static constexpr int NPO = NP | 1;                // odd row stride of the accumulator staging tile
+  static constexpr int NR = rupk(NP, 8), NN = 2 * NR, M = 128;
+  // whole cubes in a tile: an even number, so that cubes pair up
+  static constexpr int EC = M / NC / 12 * 2, EB = 6 * EC;
+  static constexpr int SL = EB;       // element slots per component (a multiple of 4)
+  static constexpr int RB = rupk(SL * NC, 8);
+  static constexpr int NPAIR = SL / 2;
+  static constexpr int NPO = NP | 1;  // odd row stride of the accumulator staging tile
   static constexpr int NCOLS = tmem_cols_for(NN);
-  static constexpr size_t A_BYTES = size_t(NN) * KA * Op::ELEM;  // one of hi / lo
-  static constexpr size_t B_BYTES = size_t(M) * KB * Op::ELEM;
-  static constexpr size_t Q_BYTES = size_t(EB) * NP * NC * 4;
-  static constexpr size_t O_BYTES = size_t(M) * NPO * 4;   // aliases the operand buffer (free by then)
-  static constexpr size_t FB_BYTES = size_t(EB) * 3 * NC * 4;
-  static constexpr size_t FN_BYTES = size_t(EB) * 4 * NC * 4;  // Fbar . n per (element, face)
-  static constexpr size_t CD_BYTES = size_t(EC) * 12 * 4;  // per cube: 6 neighbour cubes + 6 face modes
-  // per face-work entry: normal, scale, the inner neighbour's scale, packed
-  // indices; per (entry, face node): own / neighbour node, neighbour's slot
-  static constexpr size_t FR_BYTES = 24 * 8 * 4, FM_BYTES = size_t(24) * NFP * 4;
+  static constexpr size_t A_BYTES = size_t(NN) * KA * Op::ELEM;  // hi and lo
+  static constexpr size_t B_BYTES = size_t(RB) * KB * Op::ELEM;  // one of hi / lo
+  static constexpr size_t Q_BYTES = (size_t(EB) * NP * NC * 4 + 15) / 16 * 16;
+  static constexpr size_t O_BYTES = size_t(SL) * NC * NPO * 4;   // aliases the operand buffer (free by then)
+  static constexpr size_t FB_BYTES = size_t(NPAIR) * 3 * NC * 8;   // Fbar of each element pair
+  static constexpr size_t FN_BYTES = size_t(NPAIR) * 4 * NC * 8;   // 2 Fbar.n of each (element pair, face)
+  static constexpr size_t CD_BYTES = size_t(EC) * 12 * 4;        // per cube: 6 neighbour cubes + 6 face modes
+  static constexpr size_t TAB_BYTES = tc3tab_bytes(P);
   static constexpr size_t HDR = 128;
-  static constexpr size_t TAB = (sizeof(KuhnTab3<float>) + 127) / 128 * 128;
-  static constexpr size_t FIXED0 = HDR + TAB + 2 * A_BYTES + 2 * B_BYTES + FB_BYTES + FN_BYTES + CD_BYTES;
-  static constexpr size_t FIXED1 = FIXED0 + 16 + FR_BYTES + FM_BYTES;
-  // State tile buffers: two (prefetch the next tile during this one) unless
-  // a single buffer lets more blocks share an SM (228 KB of shared memory
-  // per SM, 1 KB reserved per block on sm_100a; at most 4 blocks of 256
-  // threads at the kernel's ~64 registers per thread).
+  static constexpr size_t FIXED = HDR + TAB_BYTES + A_BYTES + 2 * B_BYTES + FB_BYTES + FN_BYTES + CD_BYTES;
+  // blocks per SM that fit in shared memory (228 KB per SM, 1 KB reserved per
+  // block on sm_100a); more than four would leave too few registers
   static constexpr size_t blocks_for(size_t s) {
     return size_t(228 * 1024) / (s + 1024) < 4 ? size_t(228 * 1024) / (s + 1024) : 4;
   }
-  static constexpr int qb_for(size_t fixed) {
-    return blocks_for(fixed + Q_BYTES) > blocks_for(fixed + 2 * Q_BYTES) ? 1 : 2;
-  }
-  // the face records only where they cost neither a block per SM nor the
-  // second state buffer
-  static constexpr bool FREC = qb_for(FIXED1) >= qb_for(FIXED0) &&
-                               blocks_for(FIXED1 + qb_for(FIXED1) * Q_BYTES) >= blocks_for(FIXED0 + qb_for(FIXED0) * Q_BYTES);
-  static constexpr size_t FIXED = FREC ? FIXED1 : FIXED0;
-  static constexpr int QB = qb_for(FIXED);
-  static constexpr size_t OFF_A = HDR + TAB;
-  static constexpr size_t OFF_B = OFF_A + 2 * A_BYTES;
+  // State tile buffers: two (the next tile lands during this one, and its
+  // constant-flux phase runs behind this one's MMAs) unless the second would
+  // leave fewer than three blocks (Euler P3: three blocks and two buffers 155
+  // us at 32^3, four and one 165 us; Maxwell P4: three and one 148 us at 24^3,
+  // two and two 162 us)
+  static constexpr size_t ARGS = 256;  // batched launches: the current solve's stage arguments behind the tile
+  static constexpr size_t B1 = blocks_for(FIXED + Q_BYTES + ARGS), B2 = blocks_for(FIXED + 2 * Q_BYTES + ARGS);
+  static constexpr int QB = B2 < 3 && B1 > B2 ? 1 : 2;
+  static constexpr size_t OFF_A = HDR + TAB_BYTES;
+  static constexpr size_t OFF_B = OFF_A + A_BYTES;
   static constexpr size_t OFF_Q = OFF_B + 2 * B_BYTES;
   static constexpr size_t OFF_F = OFF_Q + QB * Q_BYTES;
   static constexpr size_t OFF_N = OFF_F + FB_BYTES;
   static constexpr size_t OFF_C = OFF_N + FN_BYTES;
-  static constexpr size_t OFF_R = (OFF_C + CD_BYTES + 15) / 16 * 16;
-  static constexpr size_t OFF_M = OFF_R + FR_BYTES;
-  static constexpr size_t SMEM = FREC ? OFF_M + FM_BYTES : OFF_C + CD_BYTES;
-  static constexpr bool BULK = (6 * NP * NC * 4) % 16 == 0;
-  static_assert(O_BYTES <= 2 * B_BYTES, "staging tile must fit the operand buffer");
+  static constexpr size_t SMEM = OFF_C + CD_BYTES;
+  // the staging tile stays off the padded volume columns, which must hold
+  // finite operand values (they meet zero operator columns) and are written
+  // by nothing else
+  static_assert(O_BYTES <= size_t(3 * NP / (Op::A_MN ? 8 : Op::CM)) * (RB / 8 * 128), "staging tile over operand padding");
+  static_assert(TAB_BYTES % 16 == 0 && SL % 4 == 0 && SL * NC <= M, "tile layout");
+  // the flux tile's last core matrices of a 128-row MMA lie inside the block's shared memory
+  static_assert(OFF_Q + size_t(M - RB) / 8 * 128 * (Op::KSTEP / (Op::A_MN ? 8 : Op::CM)) <= SMEM, "MMA reads past the tile");
   static constexpr bool FITS = SMEM + 1024 <= size_t(227 * 1024);
-  // batched launches: the current solve's stage arguments behind the tile
-  static constexpr size_t OFF_ARGS = (SMEM + 15) / 16 * 16, BATCH_SMEM = OFF_ARGS + 256;
+  static constexpr size_t OFF_ARGS = (SMEM + 15) / 16 * 16, BATCH_SMEM = OFF_ARGS + ARGS;
 };
-
-// Blocks per SM the register allocation must allow: what fits in shared
-// memory, at most three for register-light fluxes and two for the Roe /
-// HLLE / HLLEC solvers (capping those at three blocks' registers spills).
-template <class Phys, int P, class Op>
-__host__ __device__ constexpr int tc_min_blocks() {
-  return int(TcShape<P, Phys::NC, Op>::blocks_for(TcShape<P, Phys::NC, Op>::SMEM)) < (Phys::kLightFlux ? 3 : 2)
-             ? int(TcShape<P, Phys::NC, Op>::blocks_for(TcShape<P, Phys::NC, Op>::SMEM))
-             : (Phys::kLightFlux ? 3 : 2);
-}
 
 // BATCH: the tiles of many solves of one physics, order and operand kind
 // (Tc3Batch: per-tile {solve, first cell, cells}, grouped by solve; per
-// solve its stage arguments and metric table).  Each block takes a
-// contiguous range of tiles; when the solve changes, the block reloads the
-// solve's arguments (into shared memory, `args` then refers there), table
-// and face records.  A solve's tiles get exactly the arithmetic of the
-// single-solve launch, so batched results are bit-identical to it.
-// Single-solve launches pass `args0` / `tabp` and leave `bat` empty.
-template <class Phys, int P, int NT, class Op, bool BATCH>
-__global__ void __launch_bounds__(NT, tc_min_blocks<Phys, P, Op>()) stage3d_tc_kernel(
-    Stage3DArgs<float> args0, const __grid_constant__ KuhnTab3<float> tabp, Phys ph,
-    const unsigned char* __restrict__ a_image, const __grid_constant__ Tc3Batch bat) {
+// solve its stage arguments).  Each block takes a contiguous range of tiles;
+// when the solve changes, the block reloads the solve's arguments (into
+// shared memory, `args` then refers there) and table.  A solve's tiles get
+// exactly the arithmetic of the single-solve launch, so batched results are
+// bit-identical to it.  Single-solve launches pass `args0` and leave `bat`
+// empty.
+template <class Phys, int P, int NT, int MINB, class Op, bool BATCH>
+__global__ void __launch_bounds__(NT, MINB) stage3d_tc_kernel(Stage3DArgs<float> args0, Phys ph,
+                                                              const unsigned char* __restrict__ a_image,
+                                                              const __grid_constant__ Tc3Batch bat) {
   constexpr int NC = Phys::NC;
   using S = TcShape<P, NC, Op>;
-  constexpr int NP = S::NP, NFP = S::NFP, KV = S::KV, KF = S::KF, NN = S::NN, M = S::M, NPO = S::NPO;
-  constexpr int EC = S::EC, EB = S::EB, EBP = S::EBP, QV = EB * NP * NC;
+  using PP = PairPhys<Phys>;
+  constexpr int NP = S::NP, NFP = S::NFP, KV = S::KV, KF = S::KF, NN = S::NN, M = S::M, RB = S::RB, NPO = S::NPO;
+  constexpr int EC = S::EC, SL = S::SL, NPAIR = S::NPAIR, CUBE = 6 * NP * NC;
+  constexpr int QV = int(S::Q_BYTES / 4);
+  constexpr bool TWO = S::QB == 2;
+  constexpr int NEPI = (S::EB * NP + NT - 1) / NT;  // epilogue nodes per thread
   // LBO of the K-major operator image and of the flux tile (MN-major for
   // split-BF16, K-major for split-TF32); the start-address step of one MMA
   // K step in each
-  constexpr uint32_t LBO_A = NN * 16, LBO_B = umma_a_lbo<Op>(M), SBO = 128;
-  constexpr uint32_t KSTEP_A = (Op::KSTEP / Op::CM) * LBO_A, KSTEP_B = umma_a_kstep<Op>(M);
-  // byte step between the rows of consecutive components (EBP rows apart)
-  constexpr uint32_t CSTRIDE = (EBP / (Op::A_MN ? Op::CM : 8)) * 128;
+  constexpr uint32_t LBO_A = NN * 16, LBO_B = umma_a_lbo<Op>(RB), SBO = 128;
+  constexpr uint32_t KSTEP_A = (Op::KSTEP / Op::CM) * LBO_A, KSTEP_B = umma_a_kstep<Op>(RB);
   constexpr uint32_t IDESC = umma_idesc_f32acc<Op>(M, NN);
-  static_assert(NN % 16 == 0 && NN <= 256 && KV % Op::KSTEP == 0 && KF % Op::KSTEP == 0 && EC >= 1 &&
-                    EBP * NC <= M && EBP % Op::CM == 0,
+  static_assert(NN % 16 == 0 && NN <= 256 && KV % Op::KSTEP == 0 && KF % Op::KSTEP == 0 && EC >= 2 && NT % 32 == 0 &&
+                    NT >= 128,
                 "UMMA shape");
   extern __shared__ __align__(1024) unsigned char smem[];
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem);  // [0..1] q tiles, [2] mma, [3] A image
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + 32);
-  KuhnTab3<float>* tab = reinterpret_cast<KuhnTab3<float>*>(smem + S::HDR);
-  unsigned char* sAhi = smem + S::OFF_A;
-  unsigned char* sAlo = sAhi + S::A_BYTES;
+  const Tc3Tab* tab = reinterpret_cast<const Tc3Tab*>(smem + S::HDR);
+  unsigned char* sA = smem + S::OFF_A;
   unsigned char* sBhi = smem + S::OFF_B;
   unsigned char* sBlo = sBhi + S::B_BYTES;
-  float* sQ = reinterpret_cast<float*>(smem + S::OFF_Q);
-  float* sO = reinterpret_cast<float*>(sBhi);              // [M rows (c, el)][NPO], after the MMAs
-  float* sF = reinterpret_cast<float*>(smem + S::OFF_F);   // [EB][3][NC] element flux Fbar
-  float* sFn = reinterpret_cast<float*>(smem + S::OFF_N);  // [EB][4][NC] Fbar . n of each face
-  int* sNb = reinterpret_cast<int*>(smem + S::OFF_C);      // [EC][6] neighbour cube per direction
-  int* sMd = sNb + EC * 6;                                 // [EC][6] face mode | code << 8
-  float* sFR = reinterpret_cast<float*>(smem + S::OFF_R);  // [work][8] face records
-  int* sFM = reinterpret_cast<int*>(smem + S::OFF_M);      // [work][NFP] face-node indices
+  float* sQ = reinterpret_cast<float*>(smem + S::OFF_Q);  // tile states
+  float* sO = reinterpret_cast<float*>(sBhi);            // [rows (c, slot)][NPO], after the MMAs
+  f2* sF = reinterpret_cast<f2*>(smem + S::OFF_F);       // [pair][3][NC] constant flux Fbar
+  f2* sFn = reinterpret_cast<f2*>(smem + S::OFF_N);      // [pair][4][NC] 2 Fbar.n of each face
+  int2* sCd = reinterpret_cast<int2*>(smem + S::OFF_C);  // [EC][6] {neighbour cube, face mode | code << 8}
 
   // the stage arguments: the kernel parameter, or the current solve's copy
   // in shared memory (batched launches)
   Stage3DArgs<float>* sArgs = reinterpret_cast<Stage3DArgs<float>*>(smem + S::OFF_ARGS);
   const Stage3DArgs<float>& args = BATCH ? *sArgs : args0;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   grid_dep_launch();  // the next stage may set up as this one's blocks finish
   const int ngroups = BATCH ? bat.nitems : (args0.ncell - args0.cbeg + EC - 1) / EC;
   // tiles of this block: every gridDim.x-th from blockIdx.x (one solve), or
@@ -197,37 +205,13 @@ __global__ void __launch_bounds__(NT, tc_min_blocks<Phys, P, Op>()) stage3d_tc_k
     tmem_alloc(tslot, S::NCOLS);
     tmem_relinquish();
   }
-  // the solve's metric table into shared memory and its face records,
-  // decoded from the table: bits
-  // t | lf << 3 | nb_t << 5 | nb_lf << 8 | (axis + 1) << 10 | (dir > 0) << 12 | (side == 0) << 13
-  auto load_table = [&](const KuhnTab3<float>& tsrc) {
-  {
-    const int* src = reinterpret_cast<const int*>(&tsrc);
-    int* dst = reinterpret_cast<int*>(tab);
-    for (int k = tid; k < int(sizeof(KuhnTab3<float>) / 4); k += NT) dst[k] = src[k];
-  }
-  if constexpr (S::FREC) {
-  for (int w = tid; w < tsrc.n_face_work; w += NT) {
-    const int tl = tsrc.face_work[w], t = tl >> 2, lf = tl & 3;
-    const int ax = tsrc.axis[t][lf], nbt = tsrc.nb_t[t][lf], lf2 = tsrc.nb_lf[t][lf];
-    float* r = sFR + w * 8;
-    r[0] = tsrc.normal[t][lf][0];
-    r[1] = tsrc.normal[t][lf][1];
-    r[2] = tsrc.normal[t][lf][2];
-    r[3] = tsrc.fscale[t][lf];
-    r[4] = ax < 0 ? tsrc.fscale[nbt][lf2] : 0.f;
-    r[5] = __int_as_float(t | (lf << 3) | ((nbt & 7) << 5) | ((lf2 & 3) << 8) | ((ax + 1) << 10) |
-                          ((tsrc.dir[t][lf] > 0 ? 1 : 0) << 12) | ((tsrc.side[t][lf] == 0 ? 1 : 0) << 13));
-  }
-  for (int idx = tid; idx < tsrc.n_face_work * NFP; idx += NT) {
-    const int w = idx / NFP, m = idx - w * NFP;
-    const int tl = tsrc.face_work[w], t = tl >> 2, lf = tl & 3;
-    sFM[idx] = int(tsrc.own_node[lf][m]) | (int(tsrc.nb_node[t][lf][m]) << 8) | (int(tsrc.nb_m[t][lf][m]) << 16);
-  }
-  }
+  auto load_table = [&](const Tc3Tab* src) {
+    const uint4* s = reinterpret_cast<const uint4*>(src);
+    uint4* d = reinterpret_cast<uint4*>(smem + S::HDR);
+    for (int k = tid; k < int(S::TAB_BYTES / 16); k += NT) d[k] = s[k];
   };
-  if constexpr (!BATCH) load_table(tabp);
-  // zero the flux tiles once: padding rows / k columns stay zero for good
+  if constexpr (!BATCH) load_table(args0.tctab);
+  // zero the flux tiles once: padding rows / k columns stay finite for good
   for (int k = tid; k < int(2 * S::B_BYTES / 16); k += NT) reinterpret_cast<uint4*>(sBhi)[k] = make_uint4(0, 0, 0, 0);
   tc_fence_before();
   __syncthreads();
@@ -235,54 +219,66 @@ __global__ void __launch_bounds__(NT, tc_min_blocks<Phys, P, Op>()) stage3d_tc_k
   const uint32_t tmem = *tslot;
   if (tid == 0) {  // operator image (hi | lo), already in the K-major UMMA layout
     fence_proxy_async();
-    mbar_arrive_expect_tx(&bar[3], uint32_t(2 * S::A_BYTES));
-    bulk_g2s(sAhi, a_image, uint32_t(2 * S::A_BYTES), &bar[3]);
+    mbar_arrive_expect_tx(&bar[3], uint32_t(S::A_BYTES));
+    bulk_g2s(sA, a_image, uint32_t(S::A_BYTES), &bar[3]);
   }
   // the tile's state into shared memory; the tile's q_a (read by the
   // epilogue when it is not the tile's own state) into L2 at the same time
   auto issue = [&](int grp, int buf) {
     const int c0 = tile_cell0(grp), nc = tile_cells(grp);
-    const uint32_t bytes = uint32_t(nc) * 6u * NP * NC * 4u;
+    const uint32_t bytes = uint32_t(nc) * uint32_t(CUBE) * 4u;
     fence_proxy_async();
     mbar_arrive_expect_tx(&bar[buf], bytes);
     const float* qin = tile_qin(grp);
-    bulk_g2s(sQ + buf * QV, qin + size_t(c0) * 6 * NP * NC, bytes, &bar[buf]);
+    bulk_g2s(sQ + buf * QV, qin + size_t(c0) * CUBE, bytes, &bar[buf]);
     const Stage3DArgs<float>& ta = BATCH ? bat.margs[bat.items[grp].x] : args0;
-    if (!ta.rhs_only && ta.q_a != qin) bulk_prefetch_l2(ta.q_a + size_t(c0) * 6 * NP * NC, bytes);
+    if (!ta.rhs_only && ta.q_a != qin) bulk_prefetch_l2(ta.q_a + size_t(c0) * CUBE, bytes);
   };
-  // store the NC operand values v[c] of row (c, el), column k as bf16 hi / lo
-  auto put = [&](int el, int k, const float* v) {
-    const uint32_t off = umma_a_off<Op>(el, k, M);
+  // store the NC operand values v[c] of the row pair (c, slot), (c, slot + 1)
+  // (slot even), column k, as hi / lo.  Rows of consecutive components are
+  // SL apart: whole core matrices, or (SL = 4 mod 8) half a core matrix more
+  // for the odd components.
+  auto put = [&](int slot, int k, const f2* v) {
+    const uint32_t base = umma_a_off<Op>(0, k, RB);
+    const uint32_t even = base + umma_row_off<Op>(slot), odd = SL % 8 == 0 ? even : base + umma_row_off<Op>(slot + 4);
 #pragma unroll
-    for (int c = 0; c < NC; ++c) Op::put1(sBhi + off + c * CSTRIDE, sBlo + off + c * CSTRIDE, v[c]);
+    for (int c = 0; c < NC; ++c) {
+      const uint32_t off = (SL % 8 && (c & 1) ? odd : even) + uint32_t(c * SL / 8) * 128;
+      Op::put_pair(sBhi + off, sBlo + off, v[c]);
+    }
   };
-  // bit b: phase parity / copy in flight of tile buffer b (scalars, so they
-  // stay in registers)
+  // NC values of one node of two cubes
+  auto load_pair = [&](const float* a, const float* b, f2* v) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) v[c] = mk2(a[c], b[c]);
+  };
+  // bit b: phase parity / copy in flight of tile buffer b
   uint32_t par = 0u, pend = 0u, mma_parity = 0u;
   bool mma_pending = false;
   // One half of K: make the operand writes visible to the tensor-core
-  // (async) proxy, let one thread issue nks K-steps (hi*hi + hi*lo + lo*hi)
-  // against operator K-steps [ka0, ka0 + nks) (mma_issue), and wait
-  // (bounded) until they completed (mma_wait); ka0 == 0 starts the
-  // accumulator.  All threads call both.
-  auto mma_issue = [&](int ka0, int nks) {
+  // (async) proxy, let one thread issue the half's K-steps against operator
+  // K-steps from ka0 on (mma_issue), and wait (bounded) until they completed
+  // (mma_wait); ka0 == 0 starts the accumulator.  All threads call both.  A
+  // K-step is two MMAs, flux hi and flux lo against [operator hi | lo] at
+  // once (accumulator columns [0, NR) and [NR, 2 NR), added when they are
+  // read): the MMAs' fixed cost, not their size, is what the tile waits for.
+  const uint64_t desc_a = umma_desc(smem_u32(sA), LBO_A, SBO), desc_bh = umma_desc(smem_u32(sBhi), LBO_B, SBO),
+                 desc_bl = umma_desc(smem_u32(sBlo), LBO_B, SBO);
+  auto mma_issue = [&](auto ka0, auto nks) {
     fence_proxy_async();
     tc_fence_before();
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       tc_fence_after();
-      const uint32_t ah = smem_u32(sAhi), al = smem_u32(sAlo), bh = smem_u32(sBhi), bl = smem_u32(sBlo);
-#pragma unroll 1
+#pragma unroll
       for (int ks = 0; ks < nks; ++ks) {
-        const uint32_t oa = uint32_t(ka0 + ks) * KSTEP_A, ob = uint32_t(ks) * KSTEP_B;
-        const uint64_t dAh = umma_desc(ah + oa, LBO_A, SBO), dAl = umma_desc(al + oa, LBO_A, SBO);
-        const uint64_t dBh = umma_desc(bh + ob, LBO_B, SBO), dBl = umma_desc(bl + ob, LBO_B, SBO);
-        Op::mma(tmem, dBh, dAh, IDESC, (ka0 + ks) > 0 ? 1u : 0u);
-        Op::mma(tmem, dBh, dAl, IDESC, 1u);
-        Op::mma(tmem, dBl, dAh, IDESC, 1u);
+        const uint64_t da = desc_a + uint64_t((ka0 + ks) * KSTEP_A >> 4), ob = uint64_t(ks * KSTEP_B >> 4);
+        Op::mma(tmem, desc_bh + ob, da, IDESC, ka0 + ks > 0 ? 1u : 0u);
+        Op::mma(tmem, desc_bl + ob, da, IDESC, 1u);
       }
       tc_commit(&bar[2]);
     }
+    __syncwarp();
     mma_pending = true;
   };
   auto mma_wait = [&]() -> bool {
@@ -296,55 +292,62 @@ __global__ void __launch_bounds__(NT, tc_min_blocks<Phys, P, Op>()) stage3d_tc_k
   // multiples of 16 bytes (always for whole tiles of the usual shapes; the
   // last, partial tile of an odd-sized span takes plain loads).
   auto tile_bulk = [&](int g) -> bool {
-    const size_t per_cube = size_t(6) * NP * NC * 4;
+    const size_t per_cube = size_t(CUBE) * 4;
     const size_t start = reinterpret_cast<uintptr_t>(tile_qin(g)) + size_t(tile_cell0(g)) * per_cube;
     const size_t bytes = size_t(tile_cells(g)) * per_cube;
     return start % 16 == 0 && bytes % 16 == 0;
   };
-  int buf = 0;
   bool failed = !block_wait_bounded(&bar[3], 0, kWaitLimitNs);
   // the set-up above overlaps the previous stage's tail; its output (this
-  // stage's q_in / q_a / q_b, and q_out may be a buffer it still reads)
-  // only after it has completed
+  // stage's q_in / q_a, and q_out may be a buffer it still reads) only after
+  // it has completed
   grid_dep_wait();
   if (t_first < t_end && !failed && tile_bulk(t_first)) {
     if (tid == 0) issue(t_first, 0);
-    pend |= 1u;
+    pend = 1u;
   }
-  const int nwork = BATCH ? (bat.nitems > 0 ? bat.tabs[bat.items[0].x].n_face_work : 0) : tab->n_face_work;
+  int buf = 0;
   int cur_member = -1;  // batched: the solve whose arguments and table are loaded
-  // ---- per-element constant flux Fbar = F(q at node 0) and the cube-face
-  // treatment of tile g (state tile qt): one thread per (element, face); each
-  // evaluates the element's flux at node 0 (4x redundant, but the phase's
-  // latency is one flux, not four face products); the lf = 0 thread stores
-  // Fbar.  The cube-face treatment runs at the same time on threads from
-  // NT/2 on.
+  // ---- constant flux of each element of tile g (state tile qt), Fbar =
+  // F(q at node 0), and its product with the four face normals: one thread
+  // per (element pair, face), the flux evaluated by each (the phase's latency
+  // is then one flux, not four face products).  The cube-face treatment is
+  // resolved at the same time by the last threads.
   auto fbar_phase = [&](int g, const float* qt) {
     const int ncg = tile_cells(g), cg0 = tile_cell0(g);
-    for (int w = tid; w < ncg * 24; w += NT) {
-      const int el = w >> 2, lf = w & 3, t = el % 6;
-      float F[3 * NC];
-      ph.flux(&qt[el * NP * NC], F);
+    for (int w = tid; w < NPAIR * 4; w += NT) {
+      const int pr = w % NPAIR, lf = w / NPAIR, t = 2 * pr / EC, cl = 2 * pr - t * EC;
+      if (cl >= ncg) continue;
+      const float* q0 = &qt[cl * CUBE + t * NP * NC];
+      f2 qv[NC], F[3 * NC];
+      load_pair(q0, cl + 1 < ncg ? q0 + CUBE : q0, qv);
+      PP::flux(ph, qv, F);
       if (lf == 0) {
 #pragma unroll
-        for (int k = 0; k < 3 * NC; ++k) sF[el * 3 * NC + k] = F[k];
+        for (int k = 0; k < 3 * NC; ++k) sF[pr * 3 * NC + k] = F[k];
       }
-      const float nx = tab->normal[t][lf][0], ny = tab->normal[t][lf][1], nz = tab->normal[t][lf][2];
+      const f2* n3 = reinterpret_cast<const f2*>(tab->dir[t][3 + lf]);
+      const f2 two = dup2(2.0f), nx = two * n3[0], ny = two * n3[1], nz = two * n3[2];
 #pragma unroll
-      for (int c = 0; c < NC; ++c) sFn[w * NC + c] = F[c] * nx + F[NC + c] * ny + F[2 * NC + c] * nz;
+      for (int c = 0; c < NC; ++c) sFn[(pr * 4 + lf) * NC + c] = fma2(F[2 * NC + c], nz, fma2(F[NC + c], ny, F[c] * nx));
     }
-    for (int w = tid - NT / 2; w >= 0 && w < ncg * 6; w += NT / 2) {
+    for (int w = NT - 1 - tid; w < ncg * 6; w += NT) {
       const int cl = w / 6, dd = w - cl * 6;
-      cube_dirs3(cg0 + cl, args.nx, args.ny, args.nz, args.bc, sNb + cl * 6, sMd + cl * 6, dd);
+      sCd[w] = cube_dir3(cg0 + cl, args.nx, args.ny, args.nz, args.bc, dd);
     }
   };
-  // With two state buffers the next tile's copy lands while this tile is
-  // computed; its Fbar phase then runs while this tile's face MMAs do
-  // (fb_ready: sF, sFn, sNb, sMd and the tile wait are done for grp).
+  // wait (bounded) for the copy into tile buffer b
+  auto tile_wait = [&](int b) -> bool {
+    if (!block_wait_bounded(&bar[b], (par >> b) & 1u, kWaitLimitNs)) return false;
+    par ^= 1u << b;
+    pend &= ~(1u << b);
+    return true;
+  };
+  // the tile wait, sF, sFn and sCd are done for the coming tile
   bool fb_ready = false;
 
-  for (int grp = t_first; grp < t_end && !failed; grp = next_tile(grp), buf ^= (S::QB - 1)) {
-    if constexpr (BATCH) {  // a new solve: its arguments, table and face records
+  for (int grp = t_first; grp < t_end && !failed; grp = next_tile(grp), buf ^= S::QB - 1) {
+    if constexpr (BATCH) {  // a new solve: its arguments and table
       const int m = tile_member(grp);
       if (m != cur_member) {
         __syncthreads();  // every thread is done with the previous solve's tile
@@ -353,7 +356,7 @@ __global__ void __launch_bounds__(NT, tc_min_blocks<Phys, P, Op>()) stage3d_tc_k
           int* dst = reinterpret_cast<int*>(sArgs);
           for (int k = tid; k < int(sizeof(Stage3DArgs<float>) / 4); k += NT) dst[k] = src[k];
         }
-        load_table(bat.tabs[m]);
+        load_table(bat.margs[m].tctab);
         __syncthreads();
         cur_member = m;
       }
@@ -362,280 +365,307 @@ __global__ void __launch_bounds__(NT, tc_min_blocks<Phys, P, Op>()) stage3d_tc_k
     const int nc_here = tile_cells(grp);
     const int ne_here = 6 * nc_here;
     float* q = sQ + buf * QV;
-    if (fb_ready) {
-      __syncthreads();  // every thread is done with the previous tile (its buffer, sO)
-      if (S::QB == 2 && next_tile(grp) < ngroups && tile_bulk(next_tile(grp))) {
-        if (tid == 0) issue(next_tile(grp), buf ^ 1);
-        pend |= 1u << (buf ^ 1);
-      }
-    } else if (tile_bulk(grp)) {
-      if (S::QB == 1 && grp != t_first) {  // single buffer: load this tile now
-        __syncthreads();                            // every thread is done with the previous tile
-        if (tid == 0) issue(grp, 0);
-        pend |= 1u;
-      }
-      if (!block_wait_bounded(&bar[buf], (par >> buf) & 1u, kWaitLimitNs)) {
-        failed = true;
-        break;
-      }
-      par ^= 1u << buf;
-      pend &= ~(1u << buf);
-      if (S::QB == 2 && next_tile(grp) < ngroups && tile_bulk(next_tile(grp))) {
-        if (tid == 0) issue(next_tile(grp), buf ^ 1);
-        pend |= 1u << (buf ^ 1);
-      }
-    } else {
-      // plain loads; with one buffer, every thread must be done with the
-      // previous tile first
-      if (S::QB == 1) __syncthreads();
-      const float* src = args.q_in + size_t(cell0) * 6 * NP * NC;
-      for (int idx = tid; idx < ne_here * NP * NC; idx += NT) q[idx] = src[idx];
-      __syncthreads();
-    }
     if (!fb_ready) {
-      fbar_phase(grp, q);
-      __syncthreads();
-    }
-    // ---- volume fluxes (F - Fbar) in reference coordinates -> k = d*NP + j
-    // Up to five components, each thread takes two neighbouring elements
-    // (rows el, el + 1) at one node: their operand values share a 4-byte
-    // word of the MN-major tile, so each hi / lo pair is one packed
-    // conversion and one 32-bit store.  Six components (36 flux values per
-    // pair) take one element per thread.
-    if constexpr (NC > 5) {
-      for (int idx = tid; idx < EBP * NP; idx += NT) {
-        const int el8 = idx & 7, rest = idx >> 3, j = rest % NP, el = (rest / NP) * 8 + el8;
-        if (el >= ne_here) continue;
-        const int t = el % 6;
-        float F[3 * NC];
-        ph.flux(&q[(el * NP + j) * NC], F);
-        const float* Fb = &sF[el * 3 * NC];
-#pragma unroll
-        for (int k = 0; k < 3 * NC; ++k) F[k] -= Fb[k];
-        const float* iJ = tab->invJ[t];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          float v[NC];
-#pragma unroll
-          for (int c = 0; c < NC; ++c)
-            v[c] = iJ[d * 3 + 0] * F[c] + iJ[d * 3 + 1] * F[NC + c] + iJ[d * 3 + 2] * F[2 * NC + c];
-          put(el, d * NP + j, v);
+      if ((pend >> buf) & 1u) {
+        if (!tile_wait(buf)) {
+          failed = true;
+          break;
         }
+      } else {  // plain loads (one buffer: every thread is past its last read of the previous tile)
+        const float* src = args.q_in + size_t(cell0) * CUBE;
+        for (int idx = tid; idx < ne_here * NP * NC; idx += NT) q[idx] = src[idx];
+        __syncthreads();
       }
-    } else
-    for (int idx = tid; idx < (EBP / 2) * NP; idx += NT) {
-      const int e4 = idx & 3, rest = idx >> 2, j = rest % NP, el = (rest / NP) * 8 + 2 * e4;
-      if (el >= ne_here) continue;  // ne_here is even: el + 1 is in the tile too
-      const int t0 = el % 6, t1 = t0 + 1;  // el even: t0 in {0, 2, 4}
-      float Fa[3 * NC], Fb[3 * NC];
-      ph.flux(&q[(el * NP + j) * NC], Fa);
-      ph.flux(&q[((el + 1) * NP + j) * NC], Fb);
-      const float* Fba = &sF[el * 3 * NC];
+      fbar_phase(grp, q);
+    }
+    __syncthreads();  // every thread is done with the previous tile (its buffer, sO)
+    if (TWO && next_tile(grp) < ngroups && tile_bulk(next_tile(grp))) {
+      if (tid == NT / 2) issue(next_tile(grp), buf ^ 1);
+      pend |= 1u << (buf ^ 1);
+    }
+    // ---- the other traces of the cube faces (first in the work list) are
+    // gathered from global memory, one item ahead of their use; the first
+    // item's arrive behind the volume fluxes
+    constexpr int HC = EC / 2;
+    constexpr int nface_items = HC * kFaceWork3 * NFP, ncube_items = HC * kCubeFaces3 * NFP;
+    f2 go[NC];
+    auto gather = [&](int idx) {
+      const int rest = idx / HC, cl = 2 * (idx - rest * HC), wk = rest / NFP;
+      if (cl >= nc_here) return;
+      const int bits = tab->face[wk].bits, nm = tab->nodes[rest];
+      const int dd = (bits >> 12) & 7, nb = (((bits >> 5) & 7) * NP + ((nm >> 8) & 255)) * NC;
+      const float* g0 = args.q_in + size_t(sCd[cl * 6 + dd].x) * CUBE + nb;
+      const float* g1 = cl + 1 < nc_here ? args.q_in + size_t(sCd[cl * 6 + 6 + dd].x) * CUBE + nb : g0;
 #pragma unroll
-      for (int k = 0; k < 3 * NC; ++k) {
-        Fa[k] -= Fba[k];
-        Fb[k] -= Fba[3 * NC + k];
-      }
-      const float* iJa = tab->invJ[t0];
-      const float* iJb = tab->invJ[t1];
+      for (int c = 0; c < NC; ++c) go[c] = mk2(__ldg(g0 + c), __ldg(g1 + c));
+    };
+    if (tid < ncube_items) gather(tid);
+    // ---- volume fluxes (F - Fbar) in reference coordinates -> column d*NP + j.
+    // A thread keeps its element pair over its nodes, so the constant flux
+    // and the metric stay in registers (where there is room for them); PG
+    // neighbouring pairs share the 16 bytes of a core-matrix row, then come
+    // the nodes: a warp's operand stores fall in distinct banks.
+    constexpr int PG = NPAIR % 4 == 0 ? 4 : 2, TPP = NT / NPAIR;
+    static_assert(TPP >= 1, "a thread per element pair");
+    constexpr bool HOLD = NC <= 6 && MINB < 3;
+    if (tid < TPP * NPAIR) {
+      const int rest = tid / PG, pr = rest / TPP * PG + tid % PG, t = 2 * pr / EC, cl = 2 * pr - t * EC;
+      if (cl < nc_here) {
+        const f2* sFb = sF + pr * 3 * NC;
+        const f2* sG = reinterpret_cast<const f2*>(tab->dir[t]);
+        const int step = cl + 1 < nc_here ? CUBE : 0;
+        f2 Fb[HOLD ? 3 * NC : 1], G[HOLD ? 9 : 1];
+        if constexpr (HOLD) {
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const uint32_t off = umma_a_off<Op>(el, d * NP + j, M);
+          for (int k = 0; k < 3 * NC; ++k) Fb[k] = sFb[k];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          const float va = iJa[d * 3 + 0] * Fa[c] + iJa[d * 3 + 1] * Fa[NC + c] + iJa[d * 3 + 2] * Fa[2 * NC + c];
-          const float vb = iJb[d * 3 + 0] * Fb[c] + iJb[d * 3 + 1] * Fb[NC + c] + iJb[d * 3 + 2] * Fb[2 * NC + c];
-          if constexpr (Op::A_MN) {
-            Op::put2(sBhi + off + c * CSTRIDE, sBlo + off + c * CSTRIDE, va, vb);
-          } else {  // K-major: row el + 1 lies 16 bytes on, in the same core matrix (el even)
-            Op::put1(sBhi + off + c * CSTRIDE, sBlo + off + c * CSTRIDE, va);
-            Op::put1(sBhi + off + 16 + c * CSTRIDE, sBlo + off + 16 + c * CSTRIDE, vb);
+          for (int k = 0; k < 9; ++k) G[k] = sG[k];
+        }
+        for (int j = rest % TPP; j < NP; j += TPP) {
+          const float* qa = &q[cl * CUBE + (t * NP + j) * NC];
+          f2 qv[NC], F[3 * NC];
+          load_pair(qa, qa + step, qv);
+          PP::flux(ph, qv, F);
+#pragma unroll
+          for (int k = 0; k < 3 * NC; ++k) F[k] = F[k] - (HOLD ? Fb[HOLD ? k : 0] : sFb[k]);
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            const f2 gx = HOLD ? G[HOLD ? 3 * d : 0] : sG[3 * d], gy = HOLD ? G[HOLD ? 3 * d + 1 : 0] : sG[3 * d + 1],
+                     gz = HOLD ? G[HOLD ? 3 * d + 2 : 0] : sG[3 * d + 2];
+            f2 v[NC];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) v[c] = fma2(gz, F[2 * NC + c], fma2(gy, F[NC + c], gx * F[c]));
+            put(2 * pr, d * NP + j, v);
           }
         }
       }
     }
     // ---- face fluxes: (f - Fbar.n) * side*area/(6V) -> operand column lf*NFP + m
     //      (operator column KV + lf*NFP + m), into the same operand buffer.
-    // face_item evaluates work item idx into up to two operand entries
-    // (element, column, NC values); it returns how many (0: nothing to do).
-    auto face_item = [&](int idx, int& e1, int& k1, float* v1, int& e2, int& k2, float* v2) -> int {
-      const int cl = idx % EC, rest = idx / EC, m = rest % NFP, wk = rest / NFP;
+    // face_item evaluates work item idx (a face node of two cubes; cube
+    // faces with the gathered traces gn) into up to two operand entries
+    // (slot, column, NC value pairs); it returns how many (0: nothing to do).
+    auto face_item = [&](int idx, const f2* gn, int& e1, int& k1, f2* v1, int& e2, int& k2, f2* v2) -> int {
+      const int rest = idx / HC, cl = 2 * (idx - rest * HC), wk = rest / NFP, m = rest - wk * NFP;
       if (cl >= nc_here) return 0;
-      int t, lf, nbt, ax, own_n, bits = 0, nm = 0;
-      bool own_left;
-      float nx, ny, nz, scale, s2r = 0.f;
-      if constexpr (S::FREC) {
-        const float4 fr = *reinterpret_cast<const float4*>(sFR + wk * 8);
-        const float2 fr2 = *reinterpret_cast<const float2*>(sFR + wk * 8 + 4);
-        bits = __float_as_int(fr2.y);
-        nm = sFM[wk * NFP + m];
-        t = bits & 7, lf = (bits >> 3) & 3, nbt = (bits >> 5) & 7, ax = ((bits >> 10) & 3) - 1;
-        own_left = (bits >> 13) & 1;
-        own_n = nm & 255;
-        nx = fr.x, ny = fr.y, nz = fr.z, scale = fr.w, s2r = fr2.x;
-      } else {
-        const int tl = tab->face_work[wk];
-        t = tl >> 2, lf = tl & 3;
-        ax = tab->axis[t][lf];
-        own_left = tab->side[t][lf] == 0;
-        nbt = tab->nb_t[t][lf];
-        own_n = tab->own_node[lf][m];
-        nx = tab->normal[t][lf][0], ny = tab->normal[t][lf][1], nz = tab->normal[t][lf][2];
-        scale = tab->fscale[t][lf];
-      }
-      const int el = cl * 6 + t;
-      int mode = FACE_INTERIOR, code = 0, nbcube = 0;
-      if (ax >= 0) {
-        const int dd = 2 * ax + (S::FREC ? ((bits >> 12) & 1) : (tab->dir[t][lf] > 0 ? 1 : 0));
-        const int md = sMd[cl * 6 + dd];
-        mode = md & 0xff;
-        code = md >> 8;
-        nbcube = sNb[cl * 6 + dd];
-      }
-      const float* qo = &q[(el * NP + own_n) * NC];
-      float qn[NC], qg[NC];
-      if (mode == FACE_INTERIOR || mode == FACE_MIXED) {
-        const int nbn = S::FREC ? (nm >> 8) & 255 : int(tab->nb_node[t][lf][m]);
-        if (ax < 0) {
+      const int step = cl + 1 < nc_here ? CUBE : 0;
+      const Tc3Tab::Face& fr = tab->face[wk];
+      const int bits = fr.bits, nm = tab->nodes[rest];
+      const int t = bits & 7, lf = (bits >> 3) & 3;
+      const float* qo = &q[cl * CUBE + (t * NP + (nm & 255)) * NC];
+      const f2* n3 = reinterpret_cast<const f2*>(tab->dir[t][3 + lf]);
+      f2 n[3] = {n3[0], n3[1], n3[2]};
+      f2 scale = mk2(fr.scale[0], fr.scale[1]);
+      f2 L[NC], R[NC], f[NC];
+      const f2* Fn = sFn + ((t * EC + cl) / 2 * 4 + lf) * NC;
+      e1 = t * EC + cl;
+      k1 = lf * NFP + m;
+      if (idx >= ncube_items) {  // inside the cubes: side 0 is this tet, both traces are in the tile
+        const int nbt = (bits >> 5) & 7, lf2 = (bits >> 8) & 3;
+        const float* qn = &q[cl * CUBE + (nbt * NP + ((nm >> 8) & 255)) * NC];
+        load_pair(qo, qo + step, L);
+        load_pair(qn, qn + step, R);
+        f2 b[NC];
 #pragma unroll
-          for (int c = 0; c < NC; ++c) qn[c] = q[((cl * 6 + nbt) * NP + nbn) * NC + c];
-        } else {
-          const float* gq = args.q_in + ((size_t(nbcube) * 6 + nbt) * NP + nbn) * NC;
+        for (int c = 0; c < NC; ++c) b[c] = Fn[c];
+        PP::face(ph, L, R, n, b, f);
+        const f2* Fn2 = sFn + ((nbt * EC + cl) / 2 * 4 + lf2) * NC;
+        const f2 s2 = mk2(fr.scale2[0], fr.scale2[1]);
 #pragma unroll
-          for (int c = 0; c < NC; ++c) qn[c] = __ldg(gq + c);
+        for (int c = 0; c < NC; ++c) {
+          v1[c] = scale * f[c];
+          v2[c] = s2 * (f[c] + (b[c] - Fn2[c]));
         }
-      } else {
-#pragma unroll
-        for (int c = 0; c < NC; ++c) qn[c] = qo[c];
+        e2 = nbt * EC + cl;
+        k2 = lf2 * NFP + (nm >> 16);
+        return 2;
       }
-      if (mode == FACE_BC_LO) {
-        nx = -nx;
-        ny = -ny;
-        nz = -nz;
-        scale = -scale;
-      }
-      const bool bcf = mode != FACE_INTERIOR;
-      if (bcf) ph.ghost(qn, code, nx, ny, nz, qg);
-      // left/right states by value (selecting between pointers would force
-      // the register arrays into local memory)
-      float L[NC], Rr[NC];
+      const int dd = (bits >> 12) & 7;
+      const bool own_left = bits & 0x8000;
+      const int md0 = sCd[cl * 6 + dd].y, md1 = step ? sCd[cl * 6 + 6 + dd].y : md0;
+      load_pair(qo, qo + step, f);
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
-        const float o = qo[c];
-        L[c] = bcf ? qn[c] : (own_left ? o : qn[c]);
-        Rr[c] = bcf ? qg[c] : (own_left ? qn[c] : o);
+        L[c].v = own_left ? f[c].v : gn[c].v;
+        R[c].v = own_left ? gn[c].v : f[c].v;
       }
-      float f[NC];
-      ph.num_flux(L, Rr, nx, ny, nz, f);
-      // Fbar . n was taken with the table normal; a one-sided low face flips it
-      const float* Fn = &sFn[(el * 4 + lf) * NC];
-      const float sg = mode == FACE_BC_LO ? -1.f : 1.f;
+      f2 bs[NC];
 #pragma unroll
-      for (int c = 0; c < NC; ++c) v1[c] = scale * (f[c] - sg * Fn[c]);
-      e1 = el;
-      k1 = lf * NFP + m;
-      if (ax >= 0) return 1;
-      // the other tet of this inner face: same flux and normal, its own scale and Fbar
-      const int el2 = cl * 6 + nbt, lf2 = S::FREC ? (bits >> 8) & 3 : int(tab->nb_lf[t][lf]);
-      const float s2 = S::FREC ? s2r : tab->fscale[nbt][lf2];
-      const float* Fn2 = &sFn[(el2 * 4 + lf2) * NC];
+      for (int c = 0; c < NC; ++c) bs[c] = Fn[c];
+      if ((md0 | md1) & 0xff) {  // a boundary face in at least one lane
+        float l[2][NC], r[2][NC], nn[2][3], sc[2], sgn[2] = {1.0f, 1.0f};
 #pragma unroll
-      for (int c = 0; c < NC; ++c) v2[c] = s2 * (f[c] - Fn2[c]);
-      e2 = el2;
-      k2 = lf2 * NFP + (S::FREC ? (nm >> 16) : int(tab->nb_m[t][lf][m]));
-      return 2;
+        for (int c = 0; c < NC; ++c) {
+          un2(L[c], l[0][c], l[1][c]);
+          un2(R[c], r[0][c], r[1][c]);
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) un2(n[d], nn[0][d], nn[1][d]);
+        un2(scale, sc[0], sc[1]);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const int md = k ? md1 : md0, mode = md & 0xff, code = md >> 8;
+          if (mode == FACE_INTERIOR) continue;
+          // the flux is the numerical flux of (state, its ghost): the own
+          // trace, or (FACE_MIXED) the neighbour's; a one-sided low face is
+          // its element's side 0, so normal and scale flip
+          const bool from_l = (mode == FACE_MIXED) != own_left;
+          float s[NC], gh[NC];
+#pragma unroll
+          for (int c = 0; c < NC; ++c) s[c] = from_l ? l[k][c] : r[k][c];
+          if (mode == FACE_BC_LO) {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) nn[k][d] = -nn[k][d];
+            sc[k] = -sc[k];
+            sgn[k] = -1.0f;
+          }
+          ph.ghost(s, code, nn[k][0], nn[k][1], nn[k][2], gh);
+#pragma unroll
+          for (int c = 0; c < NC; ++c) {
+            l[k][c] = s[c];
+            r[k][c] = gh[c];
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          L[c] = mk2(l[0][c], l[1][c]);
+          R[c] = mk2(r[0][c], r[1][c]);
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) n[d] = mk2(nn[0][d], nn[1][d]);
+        scale = mk2(sc[0], sc[1]);
+        // Fbar . n was taken with the table normal; a one-sided low face flips it
+#pragma unroll
+        for (int c = 0; c < NC; ++c) bs[c] = bs[c] * mk2(sgn[0], sgn[1]);
+      }
+      PP::face(ph, L, R, n, bs, f);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) v1[c] = scale * f[c];
+      return 1;
     };
-    const int nface_items = EC * nwork * NFP;
     // volume half of K: operand columns [0, KV) against operator columns
     // [0, KV).  While those MMAs run, each thread evaluates its first face
     // item into registers; the operand columns are overwritten only after
     // the MMAs completed.
-    mma_issue(0, KV / Op::KSTEP);
+    mma_issue(std::integral_constant<int, 0>{}, std::integral_constant<int, KV / Op::KSTEP>{});
     int e1 = 0, k1 = 0, e2 = 0, k2 = 0;
-    float v1[NC], v2[NC];
-    const int nfirst = tid < nface_items ? face_item(tid, e1, k1, v1, e2, k2, v2) : 0;
-    if (!mma_wait()) {
-      failed = true;
-      break;
-    }
-    if (nfirst >= 1) put(e1, k1, v1);
-    if (nfirst == 2) put(e2, k2, v2);
-    for (int idx = tid + NT; idx < nface_items; idx += NT) {
-      const int n = face_item(idx, e1, k1, v1, e2, k2, v2);
-      if (n >= 1) put(e1, k1, v1);
-      if (n == 2) put(e2, k2, v2);
-    }
-    // face half of K: operand columns [0, KF) against operator columns [KV, KV + KF)
-    mma_issue(KV / Op::KSTEP, KF / Op::KSTEP);
-    // while the face MMAs run: the next tile's wait and Fbar phase (its
-    // copy was issued a whole tile earlier) ...
-    fb_ready = false;
-    if (S::QB == 2) {
-      // (a tile of another solve waits for the solve's table instead)
-      const int nxt = next_tile(grp);
-      if (nxt < ngroups && tile_bulk(nxt) && tile_member(nxt) == tile_member(grp)) {
-        if (!block_wait_bounded(&bar[buf ^ 1], (par >> (buf ^ 1)) & 1u, kWaitLimitNs)) {
+    f2 v1[NC], v2[NC];
+    for (int idx = tid;; idx += NT) {
+      int nput = 0;
+      if (idx < nface_items) {
+        f2 gn[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) gn[c] = go[c];
+        if (idx + NT < ncube_items) gather(idx + NT);
+        nput = face_item(idx, gn, e1, k1, v1, e2, k2, v2);
+      }
+      if (mma_pending) {  // (first pass of the loop)
+        if (!mma_wait()) {
           failed = true;
           break;
         }
-        par ^= 1u << (buf ^ 1);
-        pend &= ~(1u << (buf ^ 1));
+      }
+      if (nput >= 1) put(e1, k1, v1);
+      if (nput == 2) put(e2, k2, v2);
+      if (idx + NT >= nface_items) break;
+    }
+    if (failed) break;
+    // with one tile buffer: the state of this thread's epilogue nodes into
+    // registers, so that the buffer is free for the next tile from the
+    // coming barrier on
+    float vq[TWO ? 1 : NEPI][NC];
+    if constexpr (!TWO) {
+#pragma unroll
+      for (int r = 0; r < NEPI; ++r)
+        if (tid + r * NT < ne_here * NP) {
+#pragma unroll
+          for (int c = 0; c < NC; ++c) vq[r][c] = q[(tid + r * NT) * NC + c];
+        }
+    }
+    // face half of K: operand columns [0, KF) against operator columns [KV, KV + KF)
+    mma_issue(std::integral_constant<int, KV / Op::KSTEP>{}, std::integral_constant<int, KF / Op::KSTEP>{});
+    fb_ready = false;
+    const int nxt = next_tile(grp);
+    if (nxt < ngroups && tile_bulk(nxt)) {
+      if constexpr (!TWO) {  // (past the barrier: every thread is done with the tile's buffer)
+        if (tid == NT / 2) issue(nxt, 0);
+        pend = 1u;
+      } else if (tile_member(nxt) == tile_member(grp)) {
+        // while the face MMAs run: the next tile's wait and constant-flux
+        // phase (its copy was issued a whole tile earlier; a tile of another
+        // solve waits for the solve's table instead)
+        if (!tile_wait(buf ^ 1)) {
+          failed = true;
+          break;
+        }
         fbar_phase(nxt, sQ + (buf ^ 1) * QV);
         fb_ready = true;
       }
     }
-    // ... and q_a of this thread's first epilogue node (global memory when
-    // q_a is not the tile's own state)
-    const bool a_in = args.q_a == args.q_in, b_in = args.q_b == args.q_in;
-    const bool pre_a = !args.rhs_only && !a_in && tid < ne_here * NP;
-    float pa[NC];
-    if (pre_a) {
-      const size_t base = (size_t(cell0) * 6 * NP + tid) * NC;
+    // q_a of this thread's epilogue nodes (global memory when q_a is not the
+    // tile's own state), in flight behind the face MMAs
+    const bool ext_a = !args.rhs_only && args.q_a != args.q_in;
+    const size_t tile0 = size_t(cell0) * CUBE;
+    float va[NEPI][NC];
+    if (ext_a) {
 #pragma unroll
-      for (int c = 0; c < NC; ++c) pa[c] = args.q_a[base + c];
+      for (int r = 0; r < NEPI; ++r)
+        if (tid + r * NT < ne_here * NP) {
+#pragma unroll
+          for (int c = 0; c < NC; ++c) va[r][c] = args.q_a[tile0 + (tid + r * NT) * NC + c];
+        }
     }
     if (!mma_wait()) {
       failed = true;
       break;
     }
-    {  // warp w reads TMEM lanes [32 (w % 4), +32) (rows (c, el)), columns
-       // [16 (w / 4), +16) of every 16 (NT / 128) (16 at a time: bounded
-       // registers)
+    if (warp < NT / 128 * 4) {  // warp w reads TMEM lanes [32 (w % 4), +32) (rows (c, slot)), columns
+       // [8 (w / 4), +8) of every 8 (NT / 128) and their lo halves, two such groups in flight
       const int row = (warp & 3) * 32 + lane;
+      const uint32_t lanes = tmem + (uint32_t((warp & 3) * 32) << 16);
+      constexpr int STEP = 8 * (NT / 128);
 #pragma unroll
-      for (int c0 = (warp >> 2) * 16; c0 < NN; c0 += 16 * (NT / 128)) {
-        float v[16];
-        tmem_ld16(tmem + (uint32_t((warp & 3) * 32) << 16) + c0, v);
+      for (int c0 = (warp >> 2) * 8; c0 < S::NR; c0 += STEP) {
+        float v[8], w[8];
+        tmem_ld8(lanes + c0, v);
+        tmem_ld8(lanes + S::NR + c0, w);
         tmem_ld_wait();
+        if (row < SL * NC)
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-          if (c0 + i < NP) sO[row * NPO + c0 + i] = v[i];
+        for (int i = 0; i < 8; ++i)
+          if (c0 + i < NP) sO[row * NPO + c0 + i] = v[i] + w[i];
       }
     }
     tc_fence_before();
     __syncthreads();
-    // ---- epilogue per node: source, RK combine, floor, store
-    for (int idx = tid; idx < ne_here * NP; idx += NT) {
-      const int el = idx / NP, i = idx - el * NP;
-      const size_t base = (size_t(cell0) * 6 * NP + idx) * NC;
-      const float* ql = &q[idx * NC];
-      float src[NC], out[NC];
-      if (Phys::kSource) ph.source(ql, src);
+    // ---- epilogue per node: source, RK combine (every stage's q_b is its
+    // q_in), floor, store
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const float r = sO[(c * EBP + el) * NPO + i];
-        const float rhs = Phys::kSource ? r + src[c] : r;
-        if (args.rhs_only) {
-          out[c] = rhs;
-        } else {
-          const float va = a_in ? ql[c] : (pre_a && idx == tid ? pa[c] : args.q_a[base + c]);
-          const float vb = b_in ? ql[c] : args.q_b[base + c];
-          out[c] = va + args.b * (vb - va) + args.cdt * rhs;
+    for (int r = 0; r < NEPI; ++r) {
+      const int idx = tid + r * NT;
+      if (idx < ne_here * NP) {
+        const int el = idx / NP, i = idx - el * NP, cl = el / 6, slot = (el - cl * 6) * EC + cl;
+        const float* acc = sO + slot * NPO + i;
+        const float* ql = TWO ? &q[idx * NC] : vq[TWO ? 0 : r];
+        float out[NC], src[NC];
+        if constexpr (Phys::kSource) ph.source(ql, src);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          out[c] = acc[c * SL * NPO];
+          if constexpr (Phys::kSource) out[c] += src[c];
         }
-      }
-      if (Phys::kLimit && !args.rhs_only) ph.limit(out);
+        if (!args.rhs_only) {
 #pragma unroll
-      for (int c = 0; c < NC; ++c) args.q_out[base + c] = out[c];
+          for (int c = 0; c < NC; ++c) {
+            const float b = ql[c], a = ext_a ? va[r][c] : b;
+            out[c] = a + args.b * (b - a) + args.cdt * out[c];
+          }
+          if constexpr (Phys::kLimit) ph.limit(out);
+        }
+        float* dst = args.q_out + tile0 + idx * NC;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) dst[c] = out[c];
+      }
     }
   }
   if (failed) {

@@ -14,13 +14,10 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include "f32x2.cuh"
 #include "tma.cuh"
 
 namespace mxm {
-
-__host__ __device__ constexpr uint32_t umma_tile_offset(int row, int k, int rows) {
-  return uint32_t((k >> 3) * (rows >> 3) * 128 + (row >> 3) * 128 + (row & 7) * 16 + (k & 7) * 2);
-}
 
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
   uint64_t d = 0;
@@ -29,14 +26,6 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint
   d |= uint64_t((sbo >> 4) & 0x3FFFu) << 32;
   d |= uint64_t(1) << 46;  // descriptor version (sm_100)
   return d;                // base offset 0, legacy LBO mode, SWIZZLE_NONE
-}
-
-__host__ __device__ constexpr uint32_t umma_idesc_bf16_f32(int M, int N) {
-  return (1u << 4)                       // D format F32
-         | (1u << 7)                     // A format BF16
-         | (1u << 10)                    // B format BF16
-         | (uint32_t(N >> 3) << 17)      // N
-         | (uint32_t(M >> 4) << 24);     // M
 }
 
 __device__ __forceinline__ void tc_mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
@@ -59,6 +48,13 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 // Whole warp: allocate `ncols` TMEM columns (power of two >= 32); the TMEM
 // address is written to shared memory at `dst`.
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst, uint32_t ncols) {
@@ -72,33 +68,27 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
-// 32 lanes x 16 consecutive 32-bit columns: thread i of the warp receives
-// lane (warp's lane quarter + i), columns [col, col+16).
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
+// 32 lanes x 8 consecutive 32-bit columns: thread i of the warp receives
+// lane (warp's lane quarter + i), columns [col, col+8).
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
+  uint32_t r[8];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
 #pragma unroll
-  for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(r[k]);
+  for (int k = 0; k < 8; ++k) v[k] = __uint_as_float(r[k]);
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// x = hi + lo with hi, lo in bfloat16 (the split-precision operands)
-__device__ __forceinline__ void split_bf16(float x, __nv_bfloat16& hi, __nv_bfloat16& lo) {
-  hi = __float2bfloat16_rn(x);
-  lo = __float2bfloat16_rn(x - __bfloat162float(hi));
-}
-
-// Two values at once: hi and lo of (a, b) as packed bf16 pairs, a in the low
-// half (the lower address of a 4-byte word)
-__device__ __forceinline__ void split_bf16x2(float a, float b, uint32_t& hi, uint32_t& lo) {
+// Two values at once: hi and lo as packed bf16 pairs, the first lane in the
+// low half (the lower address of a 4-byte word)
+__device__ __forceinline__ void split_bf16x2(f2 v, uint32_t& hi, uint32_t& lo) {
+  float a, b;
+  un2(v, a, b);
   const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  const float2 hf = __bfloat1622float2(h);
-  const __nv_bfloat162 l = __floats2bfloat162_rn(a - hf.x, b - hf.y);
   hi = *reinterpret_cast<const uint32_t*>(&h);
+  un2(v - mk2(__uint_as_float(hi << 16), __uint_as_float(hi & 0xffff0000u)), a, b);
+  const __nv_bfloat162 l = __floats2bfloat162_rn(a, b);
   lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 
@@ -110,11 +100,6 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
   return r;
 }
-__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
-  hi = to_tf32(x);
-  lo = to_tf32(x - __uint_as_float(hi));
-}
-
 __device__ __forceinline__ void tc_mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                             uint32_t accumulate) {
   asm volatile(
@@ -142,17 +127,10 @@ struct OpBF16 {
   __device__ static void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
     tc_mma_bf16(d, a, b, idesc, acc);
   }
-  // one value: hi at ph, lo at pl
-  __device__ static void put1(unsigned char* ph, unsigned char* pl, float v) {
-    __nv_bfloat16 h, l;
-    split_bf16(v, h, l);
-    *reinterpret_cast<__nv_bfloat16*>(ph) = h;
-    *reinterpret_cast<__nv_bfloat16*>(pl) = l;
-  }
-  // two MN-adjacent values (rows r, r + 1 of one k; r even)
-  __device__ static void put2(unsigned char* ph, unsigned char* pl, float a, float b) {
+  // the values of two neighbouring rows (r even, r + 1) of one k: hi at ph, lo at pl
+  __device__ static void put_pair(unsigned char* ph, unsigned char* pl, f2 v) {
     uint32_t h, l;
-    split_bf16x2(a, b, h, l);
+    split_bf16x2(v, h, l);
     *reinterpret_cast<uint32_t*>(ph) = h;
     *reinterpret_cast<uint32_t*>(pl) = l;
   }
@@ -164,18 +142,16 @@ struct OpTF32 {
   __device__ static void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
     tc_mma_tf32(d, a, b, idesc, acc);
   }
-  __device__ static void put1(unsigned char* ph, unsigned char* pl, float v) {
-    uint32_t h, l;
-    split_tf32(v, h, l);
-    *reinterpret_cast<uint32_t*>(ph) = h;
-    *reinterpret_cast<uint32_t*>(pl) = l;
-  }
-  __device__ static void put2(unsigned char* ph, unsigned char* pl, float a, float b) {
-    uint2 h, l;
-    split_tf32(a, h.x, l.x);
-    split_tf32(b, h.y, l.y);
-    *reinterpret_cast<uint2*>(ph) = h;
-    *reinterpret_cast<uint2*>(pl) = l;
+  // rows r (even) and r + 1 are 16 bytes apart in one core matrix
+  __device__ static void put_pair(unsigned char* ph, unsigned char* pl, f2 v) {
+    float a, b;
+    un2(v, a, b);
+    const uint32_t ha = to_tf32(a), hb = to_tf32(b);
+    un2(v - mk2(__uint_as_float(ha), __uint_as_float(hb)), a, b);
+    *reinterpret_cast<uint32_t*>(ph) = ha;
+    *reinterpret_cast<uint32_t*>(ph + 16) = hb;
+    *reinterpret_cast<uint32_t*>(pl) = to_tf32(a);
+    *reinterpret_cast<uint32_t*>(pl + 16) = to_tf32(b);
   }
 };
 
@@ -207,6 +183,11 @@ __host__ __device__ constexpr uint32_t umma_k_off(int n, int k, int nn) {
 template <class Op>
 __host__ __device__ constexpr uint32_t umma_a_off(int row, int k, int rows) {
   return Op::A_MN ? umma_mn_off<Op>(row, k, rows) : umma_k_off<Op>(row, k, rows);
+}
+// the row's part of that offset (row and column parts add)
+template <class Op>
+__host__ __device__ constexpr uint32_t umma_row_off(int row) {
+  return umma_a_off<Op>(row, 0, 128);
 }
 template <class Op>
 __host__ __device__ constexpr uint32_t umma_a_lbo(int rows) {
