@@ -51,7 +51,7 @@ struct BatchGroup {
   int* d_counter = nullptr;  // [3]: one work counter per stage
   size_t smem = 0;
   int grid = 0;
-  int qv = 0, a_len = 0, aoff[6] = {0, 0, 0, 0, 0, 0};
+  int qv = 0, bv = 0, a_len = 0, aoff[6] = {0, 0, 0, 0, 0, 0};
   const void* A[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
 };
 
@@ -328,7 +328,7 @@ std::vector<int4> make_items(const Batch* b, const BatchGroup& g, const int* ec,
 void layout(const Batch* b, BatchGroup& g, const int* ec) {
   bool present[6] = {false, false, false, false, false, false};
   for (int m : g.members) present[b->members[m]->P] = true;
-  int off = 0, qv = 0, bmax = 0;
+  int off = 0, qv = 0, bmax = 0, cells = 0;
   for (int P = 1; P <= 5; ++P) {
     g.aoff[P] = 0;
     g.A[P] = nullptr;
@@ -342,10 +342,12 @@ void layout(const Batch* b, BatchGroup& g, const int* ec) {
       }
     qv = std::max(qv, 2 * ec[P] * ntri_h(P) * g.NC);
     bmax = std::max(bmax, 2 * ec[P] * bstr2d(P, g.NC, b->rbytes));
+    cells = std::max(cells, ec[P]);
   }
   g.a_len = (off + 3) / 4 * 4;
   g.qv = (qv + 3) / 4 * 4;
-  g.smem = 32 + 2 * tab_bytes(b->rbytes) + size_t(g.a_len + 2 * g.qv + bmax) * b->rbytes;
+  g.bv = (bmax + 3) / 4 * 4;
+  g.smem = 32 + 2 * tab_bytes(b->rbytes) + size_t(g.a_len + 2 * g.qv + g.bv) * b->rbytes + size_t(cells) * kCellDirs2;
 }
 
 template <class R>
@@ -363,6 +365,7 @@ Batch2DArgs<R> stage_args(const Batch* b, const BatchGroup& g, const int4* items
   }
   a.a_len = g.a_len;
   a.qv = g.qv;
+  a.bv = g.bv;
   a.err = b->derr;
   return a;
 }

@@ -48,6 +48,7 @@ struct Batch2DArgs {
   int aoff[6];        // element offset of each P's operator in the shared copy
   int a_len;          // values of all operators, a multiple of 4
   int qv;             // values per tile buffer, a multiple of 4
+  int bv;             // values of the B tile, a multiple of 4 (the cells' face treatments follow)
   int* err;
 };
 
@@ -93,6 +94,7 @@ __global__ void __launch_bounds__(NT) stage2d_batch_kernel(Batch2DArgs<R> ba, Ph
   R* sA = reinterpret_cast<R*>(smem_raw + 32 + 2 * kTabBytes);  // operators of P = 1..5
   R* sQ = sA + ba.a_len;                                          // [2][qv], 16-byte aligned
   R* sB = sQ + 2 * size_t(ba.qv);
+  int2* sCd = reinterpret_cast<int2*>(sB + ba.bv);
   const int tid = threadIdx.x;
   if (tid == 0) {
     mbar_init(&bar[0], 1);
@@ -170,11 +172,11 @@ __global__ void __launch_bounds__(NT) stage2d_batch_kernel(Batch2DArgs<R> ba, Ph
     args.err = ba.err;
     const int ne_here = 2 * item.z;
     switch (P) {
-      case 1: stage2d_tile<R, Phys, 1, NT>(args, &tabs[buf], ph, q, sB, sA + ba.aoff[1], item.y, ne_here); break;
-      case 2: stage2d_tile<R, Phys, 2, NT>(args, &tabs[buf], ph, q, sB, sA + ba.aoff[2], item.y, ne_here); break;
-      case 3: stage2d_tile<R, Phys, 3, NT>(args, &tabs[buf], ph, q, sB, sA + ba.aoff[3], item.y, ne_here); break;
-      case 4: stage2d_tile<R, Phys, 4, NT>(args, &tabs[buf], ph, q, sB, sA + ba.aoff[4], item.y, ne_here); break;
-      default: stage2d_tile<R, Phys, 5, NT>(args, &tabs[buf], ph, q, sB, sA + ba.aoff[5], item.y, ne_here); break;
+      case 1: stage2d_tile<R, Phys, 1, NT>(args, &tabs[buf], ph, q, sB, sA + ba.aoff[1], sCd, item.y, ne_here); break;
+      case 2: stage2d_tile<R, Phys, 2, NT>(args, &tabs[buf], ph, q, sB, sA + ba.aoff[2], sCd, item.y, ne_here); break;
+      case 3: stage2d_tile<R, Phys, 3, NT>(args, &tabs[buf], ph, q, sB, sA + ba.aoff[3], sCd, item.y, ne_here); break;
+      case 4: stage2d_tile<R, Phys, 4, NT>(args, &tabs[buf], ph, q, sB, sA + ba.aoff[4], sCd, item.y, ne_here); break;
+      default: stage2d_tile<R, Phys, 5, NT>(args, &tabs[buf], ph, q, sB, sA + ba.aoff[5], sCd, item.y, ne_here); break;
     }
     buf ^= 1;
   }

@@ -198,6 +198,27 @@ void fill_tab2(Handle* h, KuhnTab2<R>& t) {
     }
   for (int lf = 0; lf < 3; ++lf)
     for (int m = 0; m < h->NFP; ++m) t.own_node[lf][m] = uint8_t(h->ref.face_nodes[((lf + 2) % 3) * h->NFP + m]);
+  // faces a cell evaluates once, the cell faces before the diagonal
+  int n = 0;
+  for (int inner = 0; inner < 2; ++inner)
+    for (int a = 0; a < 2; ++a)
+      for (int lf = 0; lf < 3; ++lf) {
+        const int ax = k.axis[a][lf], nbt = k.nb_t[a][lf], lf2 = k.nb_lf[a][lf];
+        if ((ax < 0) != (inner == 1) || (inner && k.side[a][lf] != 0)) continue;
+        if (n == 5) throw ArgError("internal: Kuhn face work list");
+        for (int d = 0; d < 2; ++d)
+          if (k.off[a][lf][d] != (d == ax ? k.dir[a][lf] : 0)) throw ArgError("internal: cell face offset");
+        t.fbits[n] = a | (lf << 1) | (nbt << 3) | (lf2 << 4) |
+                     (ax >= 0 ? (2 * ax + (k.dir[a][lf] > 0 ? 1 : 0)) << 6 : 0x200) | (k.side[a][lf] == 0 ? 0x100 : 0);
+        for (int m = 0; m < h->NFP; ++m) {
+          int mm = 0;
+          while (mm < h->NFP && t.own_node[lf2][mm] != t.nb_node[a][lf][m]) ++mm;
+          if (mm == h->NFP) throw ArgError("internal: neighbour face node not found");
+          t.fnode[n][m] = int(t.own_node[lf][m]) | (int(t.nb_node[a][lf][m]) << 8) | (mm << 16);
+        }
+        ++n;
+      }
+  if (n != 5) throw ArgError("internal: Kuhn face work list");
   for (int a = 0; a < 2; ++a)
     for (int q = 0; q < 4; ++q) t.invJ[a][q] = R(k.invJ[a][q]);
 }

@@ -68,6 +68,12 @@ struct KuhnTab2 {
   int8_t dir[2][3];
   uint8_t own_node[3][kMaxNFP2];
   uint8_t nb_node[2][3][kMaxNFP2];
+  // faces a cell evaluates once: its four cell faces, then the diagonal (by
+  // its side-0 triangle).  Bits t | lf << 1 | nb_t << 3 | nb_lf << 4 |
+  // (2 axis + (dir > 0)) << 6 (cell faces) | (side == 0) << 8 | axis < 0 << 9;
+  // nodes own | neighbour's << 8 | neighbour's face index << 16
+  int32_t fbits[5];
+  int32_t fnode[5][kMaxNFP2];
 };
 
 // Dynamic shared memory one block may use on sm_100a.
@@ -153,6 +159,15 @@ __device__ __forceinline__ int2 cube_dir3(int cell, int nx, int ny, int nz, cons
   const int ni = ax == 0 ? wrapi(ci + dir, nx) : ci, nj = ax == 1 ? wrapi(cj + dir, ny) : cj,
             nk = ax == 2 ? wrapi(ck + dir, nz) : ck;
   return make_int2(ni + nx * (nj + ny * nk), mode | (code << 8));
+}
+
+// The same for one of the four faces of a 2D cell.
+__device__ __forceinline__ int2 cell_dir2(int cell, int nx, int ny, const int* bc, int dd) {
+  const int cj = div_cells(cell, nx), ci = cell - cj * nx, ax = dd >> 1, dir = (dd & 1) ? 1 : -1;
+  int code;
+  const int mode = face_mode(ax, dir, ax == 0 ? ci : cj, ax == 0 ? nx : ny, bc, code);
+  const int ni = ax == 0 ? wrapi(ci + dir, nx) : ci, nj = ax == 1 ? wrapi(cj + dir, ny) : cj;
+  return make_int2(nj * nx + ni, mode | (code << 8));
 }
 
 // Resident blocks per SM of a persistent kernel with `nt` threads and `smem`

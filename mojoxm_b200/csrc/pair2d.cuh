@@ -1,0 +1,224 @@
+// Lane forms of the 2D physics: the 2D stage evaluates the fluxes of the same
+// node of LN neighbouring cells at once -- two in packed FP32 (f2), one in
+// FP64 -- with the indices, metric terms and normals shared by the lanes.
+#pragma once
+#include <type_traits>
+
+#include "f32x2.cuh"
+#include "pair.cuh"
+#include "physics2d.cuh"
+
+namespace mxm {
+
+// arithmetic common to double and f2
+__device__ __forceinline__ double fma2(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ double max2(double a, double b) { return a > b ? a : b; }
+__device__ __forceinline__ double min2(double a, double b) { return a < b ? a : b; }
+__device__ __forceinline__ double abs2(double a) { return fabs(a); }
+__device__ __forceinline__ double absadd2(double a, double b) { return fabs(a) + b; }
+__device__ __forceinline__ double rcp2(double a) { return 1.0 / a; }
+__device__ __forceinline__ double sqrt2(double a) { return sqrt(a); }
+// x / y with y positive: FP64 the quotient; FP32 a reciprocal and one
+// residual step, which brings it within an ulp of the quotient
+__device__ __forceinline__ double quot2(double x, double y, double) { return x / y; }
+__device__ __forceinline__ f2 quot2(f2 x, f2 y, f2 ri) {
+  const f2 k = x * ri;
+  return fma2(fma2(k * dup2(-1.0f), y, x), ri, k);
+}
+
+template <class R>
+struct Lanes;
+template <>
+struct Lanes<float> {
+  static constexpr int LN = 2;
+  using T = f2;
+  __device__ static f2 dup(float a) { return dup2(a); }
+  __device__ static f2 make(const float* a) { return mk2(a[0], a[1]); }
+  __device__ static void split(f2 x, float* a) { un2(x, a[0], a[1]); }
+};
+template <>
+struct Lanes<double> {
+  static constexpr int LN = 1;
+  using T = double;
+  __device__ static double dup(double a) { return a; }
+  __device__ static double make(const double* a) { return a[0]; }
+  __device__ static void split(double x, double* a) { a[0] = x; }
+};
+
+// Any 2D physics: its scalar functions once per lane.
+template <class R, class Phys>
+struct ScalarLanes2 {
+  using V = Lanes<R>;
+  using T = typename V::T;
+  static constexpr int NC = Phys::NC, LN = V::LN;
+  __device__ __forceinline__ static void flux(const Phys& ph, const T* q, T* Fx, T* Fy) {
+    R s[NC][LN], x[NC][LN], y[NC][LN];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) V::split(q[c], s[c]);
+#pragma unroll
+    for (int k = 0; k < LN; ++k) {
+      R v[NC], fx[NC], fy[NC];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) v[c] = s[c][k];
+      ph.flux(v, fx, fy);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        x[c][k] = fx[c];
+        y[c][k] = fy[c];
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      Fx[c] = V::make(x[c]);
+      Fy[c] = V::make(y[c]);
+    }
+  }
+  __device__ __forceinline__ static void face(const Phys& ph, const T* l, const T* r, T nx, T ny, T* f) {
+    R a[NC][LN], b[NC][LN], o[NC][LN], n[2][LN];
+    V::split(nx, n[0]);
+    V::split(ny, n[1]);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      V::split(l[c], a[c]);
+      V::split(r[c], b[c]);
+    }
+#pragma unroll
+    for (int k = 0; k < LN; ++k) {
+      R x[NC], y[NC], g[NC];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        x[c] = a[c][k];
+        y[c] = b[c][k];
+      }
+      ph.face(x, y, n[0][k], n[1][k], g);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) o[c][k] = g[c];
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) f[c] = V::make(o[c]);
+  }
+  // face() out of line and by value, for a rare branch: inlined, its
+  // registers would be every caller's
+  struct Vec {
+    T v[NC];
+  };
+  __device__ __noinline__ static Vec face_call(const Phys ph, const Vec l, const Vec r, T nx, T ny) {
+    Vec o;
+    face(ph, l.v, r.v, nx, ny, o.v);
+    return o;
+  }
+};
+
+// Euler, Rusanov and HLLE (src/local_mesh_2d_gpu_euler.mojo:33-337; HLLE is
+// the 3D solver on the embedded state, src/euler.mojo:364-412, whose
+// face-frame rotation and third momentum drop out here).
+template <class R, int FLUX>
+struct EulerLanes2 {
+  using V = Lanes<R>;
+  using T = typename V::T;
+  using Phys = Euler2D<R, FLUX>;
+  struct Pre {
+    T rho, u, v, p, ri;
+  };
+  __device__ __forceinline__ static void pre(const Phys& ph, const T* q, Pre& a) {
+    a.rho = max2(q[0], ph.rho_min);
+    a.ri = rcp2(a.rho);
+    a.u = quot2(q[1], a.rho, a.ri);
+    a.v = quot2(q[2], a.rho, a.ri);
+    const T ke = fma2(q[2], a.v, q[1] * a.u);
+    a.p = max2(fma2(ke, V::dup(R(-0.5)), q[3]) * V::dup(ph.gamma - R(1)), ph.p_min);
+  }
+  __device__ __forceinline__ static void flux(const Phys& ph, const T* q, T* Fx, T* Fy) {
+    Pre a;
+    pre(ph, q, a);
+    const T H = q[3] + a.p;
+    Fx[0] = q[1], Fx[1] = fma2(q[1], a.u, a.p), Fx[2] = q[1] * a.v, Fx[3] = a.u * H;
+    Fy[0] = q[2], Fy[1] = Fx[2], Fy[2] = fma2(q[2], a.v, a.p), Fy[3] = a.v * H;
+  }
+  __device__ __forceinline__ static void face(const Phys& ph, const T* l, const T* r, T nx, T ny, T* f) {
+    if (FLUX == FLUX_HLLE && ph.entropy_fix) {
+      using One = ScalarLanes2<R, Phys>;
+      typename One::Vec x, y;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) x.v[k] = l[k], y.v[k] = r[k];
+      const typename One::Vec o = One::face_call(ph, x, y, nx, ny);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) f[k] = o.v[k];
+      return;
+    }
+    Pre x, y;
+    pre(ph, l, x);
+    pre(ph, r, y);
+    const T ga = V::dup(ph.gamma), h = V::dup(R(0.5));
+    const T mnl = fma2(l[2], ny, l[1] * nx), mnr = fma2(r[2], ny, r[1] * nx);
+    const T ul = mnl * x.ri, ur = mnr * y.ri, cl = sqrt2(ga * x.p * x.ri), cr = sqrt2(ga * y.p * y.ri);
+    T al, be;
+    if constexpr (FLUX == FLUX_HLLE) {
+      const T il = sqrt2(x.ri), ir = sqrt2(y.ri), is = rcp2(fma2(x.rho, il, y.rho * ir)), wl = il * is, wr = ir * is;
+      const T vx = fma2(l[1], wl, r[1] * wr), vy = fma2(l[2], wl, r[2] * wr);
+      const T H = fma2(l[3] + x.p, wl, (r[3] + y.p) * wr), v2 = fma2(vy, vy, vx * vx);
+      const T c = sqrt2(max2(fma2(v2, V::dup(R(-0.5)), H) * V::dup(ph.gamma - R(1)), R(0)));
+      const T u = fma2(vy, ny, vx * nx), s0 = min2(ul - cl, u - c), s2 = max2(ur + cr, u + c);
+      // sum_k |s_k| W_k = al (fr - fl) + be (r - l)
+      const T a0 = abs2(s0), a2 = abs2(s2), iden = rcp2(s2 - s0);
+      al = (a2 - a0) * iden;
+      be = (a0 * s2 - a2 * s0) * iden;
+    } else {
+      be = max2(sqrt2(fma2(x.v, x.v, x.u * x.u)) + cl, sqrt2(fma2(y.v, y.v, y.u * y.u)) + cr);
+    }
+    auto comp = [&](int k, T fl, T fr) {
+      T d = be * (r[k] - l[k]);
+      if constexpr (FLUX == FLUX_HLLE) d = fma2(al, fr - fl, d);
+      f[k] = h * ((fl + fr) - d);
+    };
+    comp(0, mnl, mnr);
+    comp(1, fma2(l[1], ul, x.p * nx), fma2(r[1], ur, y.p * nx));
+    comp(2, fma2(l[2], ul, x.p * ny), fma2(r[2], ur, y.p * ny));
+    comp(3, (l[3] + x.p) * ul, (r[3] + y.p) * ur);
+  }
+};
+template <class R, class Phys>
+struct Phys2 : ScalarLanes2<R, Phys> {};
+template <class R>
+struct Phys2<R, Euler2D<R, FLUX_HLLE>> : EulerLanes2<R, FLUX_HLLE> {};
+template <class R>
+struct Phys2<R, Euler2D<R, FLUX_RUSANOV>> : EulerLanes2<R, FLUX_RUSANOV> {};
+
+// Shallow water, Rusanov (src/local_mesh_2d_gpu_sw.mojo:27-306).
+template <class R>
+struct Phys2<R, ShallowWater2D<R, FLUX_RUSANOV>> {
+  using V = Lanes<R>;
+  using T = typename V::T;
+  using Phys = ShallowWater2D<R, FLUX_RUSANOV>;
+  struct Pre {
+    T h, u, v, p;
+  };
+  __device__ __forceinline__ static void pre(const Phys& ph, const T* q, Pre& a) {
+    a.h = max2(q[0], ph.h_min);
+    const T ri = rcp2(a.h);
+    a.u = quot2(q[1], a.h, ri);
+    a.v = quot2(q[2], a.h, ri);
+    a.p = V::dup(R(0.5) * ph.g) * a.h * a.h;
+  }
+  __device__ __forceinline__ static void flux(const Phys& ph, const T* q, T* Fx, T* Fy) {
+    Pre a;
+    pre(ph, q, a);
+    Fx[0] = q[1], Fx[1] = fma2(q[1], a.u, a.p), Fx[2] = q[1] * a.v;
+    Fy[0] = q[2], Fy[1] = Fx[2], Fy[2] = fma2(q[2], a.v, a.p);
+  }
+  __device__ __forceinline__ static void face(const Phys& ph, const T* l, const T* r, T nx, T ny, T* f) {
+    Pre x, y;
+    pre(ph, l, x);
+    pre(ph, r, y);
+    const T h = V::dup(R(0.5)), g = V::dup(ph.g);
+    const T al = max2(sqrt2(fma2(x.v, x.v, x.u * x.u)) + sqrt2(g * x.h), sqrt2(fma2(y.v, y.v, y.u * y.u)) + sqrt2(g * y.h));
+    const T ml = fma2(l[2], ny, l[1] * nx), mr = fma2(r[2], ny, r[1] * nx);
+    const T ul = fma2(x.v, ny, x.u * nx), ur = fma2(y.v, ny, y.u * nx);
+    auto comp = [&](int k, T fl, T fr) { f[k] = h * ((fl + fr) - al * (r[k] - l[k])); };
+    comp(0, ml, mr);
+    comp(1, fma2(l[1], ul, x.p * nx), fma2(r[1], ur, y.p * nx));
+    comp(2, fma2(l[2], ul, x.p * ny), fma2(r[2], ur, y.p * ny));
+  }
+};
+
+}  // namespace mxm

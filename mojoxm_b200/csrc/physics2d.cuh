@@ -1,6 +1,6 @@
 // Device physics of mojoxm's 2D triangle kernels.  Unlike 3D these are not
 // routed through the Physics trait: each has its own volume-flux floors and
-// face-flux formula (ghost states built inside the face kernel).
+// face-flux formula; a boundary face is the interior flux of (trace, ghost).
 //   Euler   src/local_mesh_2d_gpu_euler.mojo:33-144 (vol), :220-337 (Rusanov,
 //           alpha = |v| + c), :392-545 (HLLC); HLLE = the 3D euler_hlle_solver on
 //           the state embedded with w = 0, n_z = 0 (src/euler.mojo:364-412)
@@ -24,12 +24,10 @@ struct Advection2D {
     Fx[0] = vx * q[0];
     Fy[0] = vy * q[0];
   }
-  __device__ void face(const R* qL, const R* qR, int bc, R nx, R ny, R* f) const {
-    R vn = vx * nx + vy * ny;
-    if (vn >= R(0)) f[0] = vn * qL[0];
-    else if (bc == BC_INTERIOR) f[0] = vn * qR[0];
-    else if (bc == BC_INFLOW) f[0] = vn * inflow_q;
-    else f[0] = R(0);
+  __device__ void ghost(const R*, int bc, R, R, R* g) const { g[0] = bc == BC_INFLOW ? inflow_q : R(0); }
+  __device__ void face(const R* qL, const R* qR, R nx, R ny, R* f) const {
+    const R vn = vx * nx + vy * ny;
+    f[0] = vn * (vn >= R(0) ? qL[0] : qR[0]);
   }
   __device__ void source(const R*, R* s) const { s[0] = R(0); }
   __device__ R speed(const R*) const { return sqrt(vx * vx + vy * vy); }
@@ -61,10 +59,7 @@ struct Euler2D {
       g[0] = qL[0]; g[1] = qL[1]; g[2] = qL[2]; g[3] = qL[3];
     }
   }
-  __device__ void face(const R* qL, const R* qRin, int bc, R nx, R ny, R* f) const {
-    R qR[4];
-    if (bc == BC_INTERIOR) { qR[0] = qRin[0]; qR[1] = qRin[1]; qR[2] = qRin[2]; qR[3] = qRin[3]; }
-    else ghost(qL, bc, nx, ny, qR);
+  __device__ void face(const R* qL, const R* qR, R nx, R ny, R* f) const {
     if (FLUX == FLUX_HLLE) {
       EulerD<R, FLUX_HLLE> e3;
       e3.gamma = gamma; e3.rho_min = rho_min; e3.p_min = p_min; e3.entropy_fix = entropy_fix;
@@ -160,14 +155,16 @@ struct ShallowWater2D {
     Fx[0] = q[1]; Fx[1] = q[1] * u + p; Fx[2] = q[1] * v;
     Fy[0] = q[2]; Fy[1] = q[2] * u; Fy[2] = q[2] * v + p;
   }
-  __device__ void face(const R* qL, const R* qRin, int bc, R nx, R ny, R* f) const {
-    R qR[3];
-    if (bc == BC_INTERIOR) { qR[0] = qRin[0]; qR[1] = qRin[1]; qR[2] = qRin[2]; }
-    else if (bc == BC_WALL) {
-      R mn = qL[1] * nx + qL[2] * ny;
-      qR[0] = qL[0]; qR[1] = qL[1] - R(2) * mn * nx; qR[2] = qL[2] - R(2) * mn * ny;
-    } else if (bc == BC_INFLOW) { qR[0] = inflow[0]; qR[1] = inflow[1]; qR[2] = inflow[2]; }
-    else { qR[0] = qL[0]; qR[1] = qL[1]; qR[2] = qL[2]; }
+  __device__ void ghost(const R* q, int bc, R nx, R ny, R* g) const {
+    if (bc == BC_WALL) {
+      const R mn = q[1] * nx + q[2] * ny;
+      g[0] = q[0]; g[1] = q[1] - R(2) * mn * nx; g[2] = q[2] - R(2) * mn * ny;
+    } else {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) g[k] = bc == BC_INFLOW ? inflow[k] : q[k];
+    }
+  }
+  __device__ void face(const R* qL, const R* qR, R nx, R ny, R* f) const {
     R hL = qL[0] < h_min ? h_min : qL[0], hR = qR[0] < h_min ? h_min : qR[0];
     R uL = qL[1] / hL, vL = qL[2] / hL, uR = qR[1] / hR, vR = qR[2] / hR;
     R pL = R(0.5) * g * hL * hL, pR = R(0.5) * g * hR * hR;
@@ -223,22 +220,17 @@ struct Maxwell2D {
     Fx[0] = R(0); Fx[1] = c2 * q[5]; Fx[2] = -c2 * q[4]; Fx[3] = R(0); Fx[4] = -q[2]; Fx[5] = q[1];
     Fy[0] = -c2 * q[5]; Fy[1] = R(0); Fy[2] = c2 * q[3]; Fy[3] = q[2]; Fy[4] = R(0); Fy[5] = -q[0];
   }
-  __device__ void face(const R* qL, const R* qRin, int bc, R nx, R ny, R* f) const {
-    R qR[6];
-    if (bc == BC_INTERIOR) {
-#pragma unroll
-      for (int k = 0; k < 6; ++k) qR[k] = qRin[k];
-    } else if (bc == BC_WALL) {
-      R En = qL[0] * nx + qL[1] * ny, Bn = qL[3] * nx + qL[4] * ny;
-      qR[0] = R(2) * En * nx - qL[0]; qR[1] = R(2) * En * ny - qL[1]; qR[2] = -qL[2];
-      qR[3] = qL[3] - R(2) * Bn * nx; qR[4] = qL[4] - R(2) * Bn * ny; qR[5] = qL[5];
-    } else if (bc == BC_INFLOW) {
-#pragma unroll
-      for (int k = 0; k < 6; ++k) qR[k] = inflow[k];
+  __device__ void ghost(const R* q, int bc, R nx, R ny, R* g) const {
+    if (bc == BC_WALL) {
+      const R En = q[0] * nx + q[1] * ny, Bn = q[3] * nx + q[4] * ny;
+      g[0] = R(2) * En * nx - q[0]; g[1] = R(2) * En * ny - q[1]; g[2] = -q[2];
+      g[3] = q[3] - R(2) * Bn * nx; g[4] = q[4] - R(2) * Bn * ny; g[5] = q[5];
     } else {
 #pragma unroll
-      for (int k = 0; k < 6; ++k) qR[k] = qL[k];
+      for (int k = 0; k < 6; ++k) g[k] = bc == BC_INFLOW ? inflow[k] : q[k];
     }
+  }
+  __device__ void face(const R* qL, const R* qR, R nx, R ny, R* f) const {
     R c2 = c * c, h = R(0.5);
     f[0] = h * (c2 * (-qL[5] * ny) + c2 * (-qR[5] * ny)) - h * c * (qR[0] - qL[0]);
     f[1] = h * (c2 * (qL[5] * nx) + c2 * (qR[5] * nx)) - h * c * (qR[1] - qL[1]);
@@ -292,23 +284,18 @@ struct Mhd2D {
     return sp;
   }
   __device__ void flux(const R* q, R* Fx, R* Fy) const { (void)flux_speed(q, Fx, Fy); }
-  __device__ void face(const R* qL, const R* qRin, int bc, R nx, R ny, R* f) const {
-    R qR[NC];
-    if (bc == BC_INTERIOR) {
-#pragma unroll
-      for (int k = 0; k < NC; ++k) qR[k] = qRin[k];
-    } else if (bc == BC_WALL) {  // conducting slip wall: reflect m_n and B_n (GLM: psi too)
-      const R mn = qL[1] * nx + qL[2] * ny, bn = qL[3] * nx + qL[4] * ny;
-      qR[0] = qL[0]; qR[1] = qL[1] - R(2) * mn * nx; qR[2] = qL[2] - R(2) * mn * ny;
-      qR[3] = qL[3] - R(2) * bn * nx; qR[4] = qL[4] - R(2) * bn * ny; qR[5] = qL[5];
-      if (GLM) qR[NC - 1] = -qL[NC - 1];
-    } else if (bc == BC_INFLOW) {
-#pragma unroll
-      for (int k = 0; k < NC; ++k) qR[k] = inflow[k];
+  __device__ void ghost(const R* q, int bc, R nx, R ny, R* g) const {
+    if (bc == BC_WALL) {  // conducting slip wall: reflect m_n and B_n (GLM: psi too)
+      const R mn = q[1] * nx + q[2] * ny, bn = q[3] * nx + q[4] * ny;
+      g[0] = q[0]; g[1] = q[1] - R(2) * mn * nx; g[2] = q[2] - R(2) * mn * ny;
+      g[3] = q[3] - R(2) * bn * nx; g[4] = q[4] - R(2) * bn * ny; g[5] = q[5];
+      if (GLM) g[NC - 1] = -q[NC - 1];
     } else {
 #pragma unroll
-      for (int k = 0; k < NC; ++k) qR[k] = qL[k];
+      for (int k = 0; k < NC; ++k) g[k] = bc == BC_INFLOW ? inflow[k] : q[k];
     }
+  }
+  __device__ void face(const R* qL, const R* qR, R nx, R ny, R* f) const {
     R FxL[NC], FyL[NC], FxR[NC], FyR[NC];
     const R sL = flux_speed(qL, FxL, FyL), sR = flux_speed(qR, FxR, FyR);
     const R al = sL > sR ? sL : sR, h = R(0.5);

@@ -17,6 +17,7 @@
 // (batch2d.cuh).
 #pragma once
 #include "dg_common.cuh"
+#include "pair2d.cuh"
 #include "physics2d.cuh"
 #include "tma.cuh"
 
@@ -31,7 +32,7 @@ struct Stage2DShape {
   static constexpr int BSTR = BSTR_RAW + ((1 - BSTR_RAW % BMOD) + BMOD) % BMOD;
   // rows of the contraction per thread: a divisor of NP
   static constexpr int RI = P == 1 ? 1 : (P == 2 ? 2 : (P == 3 ? 2 : (P == 4 ? 3 : 3)));
-  static constexpr size_t kPerCell = 2 * sizeof(R) * (2 * size_t(NP) * NC + BSTR);  // 2 q buffers + B rows
+  static constexpr size_t kPerCell = 2 * sizeof(R) * (2 * size_t(NP) * NC + BSTR) + 32;  // 2 q buffers, B rows, face treatments
 };
 
 constexpr uint64_t kWaitLimitNs2 = 2000000000ull;
@@ -53,81 +54,155 @@ __device__ __forceinline__ void load_node(const R* p, R* v) {
   }
 }
 
+// Shared memory of a tile's cell-face treatments.
+constexpr int kCellDirs2 = 4 * int(sizeof(int2));
+
 // One tile of whole cells starting at cell0 (ne_here triangles), its state
 // already in shared memory at q: volume and edge fluxes into sB, then
-// rhs = A B + source and the RK combine into args.q_out.  Contains one
-// block barrier; every thread of the block must call it.
+// rhs = A B + source and the RK combine into args.q_out.  Contains block
+// barriers; every thread of the block must call it.
+//
+// Bound by its instruction stream (the contraction is 4 % of it), so: the
+// fluxes of the same node of two neighbouring cells go through packed FP32
+// arithmetic (FP64: one cell a thread); the diagonal is evaluated once for
+// both triangles; the neighbour and boundary treatment of each cell face is
+// resolved once per tile (sCd) instead of by an integer division and half a
+// dozen table bytes per face node; HLLE works in the world frame on the two
+// momenta instead of on the state embedded in 3D.  Shallow water P3, 181^2
+// cells: 23.7 -> 16.8 us a stage.
 template <class R, class Phys, int P, int NT>
 __device__ __forceinline__ void stage2d_tile(const Stage2DArgs<R>& args, const KuhnTab2<R>* tab, const Phys& ph,
-                                             const R* q, R* sB, const R* sA, int cell0, int ne_here) {
+                                             const R* q, R* sB, const R* sA, int2* sCd, int cell0, int ne_here) {
   constexpr int NC = Phys::NC;
   using S = Stage2DShape<P, NC, R>;
-  constexpr int NP = S::NP, NFP = S::NFP, K = S::K, BSTR = S::BSTR, NS = S::NS, RI = S::RI, G = NP / RI;
+  using V = Lanes<R>;
+  using T = typename V::T;
+  using P2 = Phys2<R, Phys>;
+  constexpr int NP = S::NP, NFP = S::NFP, K = S::K, BSTR = S::BSTR, NS = S::NS, RI = S::RI, G = NP / RI, LN = V::LN;
   static_assert(NP % RI == 0, "row tile must divide NP");
-  const int tid = threadIdx.x;
-  for (int idx = tid; idx < ne_here * NP; idx += NT) {
-    const int el = idx / NP, j = idx - el * NP, t = el & 1;
-    R Fx[NC], Fy[NC], qv[NC];
-    load_node<NC>(&q[(el * NP + j) * NC], qv);
-    ph.flux(qv, Fx, Fy);
+  const int tid = threadIdx.x, nc_here = ne_here / 2, npair = (nc_here + LN - 1) / LN;
+  // NC values of one node of LN cells, and their store into LN rows of sB
+  auto load = [&](const R* const* p, T* v) {
+    R x[LN][NC];
+#pragma unroll
+    for (int k = 0; k < LN; ++k) load_node<NC>(p[k], x[k]);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      R y[LN];
+#pragma unroll
+      for (int k = 0; k < LN; ++k) y[k] = x[k][c];
+      v[c] = V::make(y);
+    }
+  };
+  auto put = [&](R* b, int step, const T* v) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      R y[LN];
+      V::split(v[c], y);
+#pragma unroll
+      for (int k = 0; k < LN; ++k) b[k * step + c] = y[k];
+    }
+  };
+  for (int w = tid; w < nc_here * 4; w += NT) sCd[w] = cell_dir2(cell0 + (w >> 2), args.nx, args.ny, args.bc, w & 3);
+  for (int idx = tid; idx < npair * 2 * NP; idx += NT) {
+    const int rest = idx / NP, j = idx - rest * NP, t = rest & 1, cl = (rest >> 1) * LN, el = cl * 2 + t;
+    const int up = cl + 1 < nc_here ? 2 : 0;  // the second lane's element (the first again past the tile's end)
+    const R* p[LN];
+#pragma unroll
+    for (int k = 0; k < LN; ++k) p[k] = &q[((el + k * up) * NP + j) * NC];
+    T qv[NC], Fx[NC], Fy[NC], br[NC], bs[NC];
+    load(p, qv);
+    P2::flux(ph, qv, Fx, Fy);
     const R* iJ = tab->invJ[t];
+    const T i0 = V::dup(iJ[0]), i1 = V::dup(iJ[1]), i2 = V::dup(iJ[2]), i3 = V::dup(iJ[3]);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      br[c] = fma2(i1, Fy[c], i0 * Fx[c]);
+      bs[c] = fma2(i3, Fy[c], i2 * Fx[c]);
+    }
     R* b = &sB[el * BSTR + j * NS];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      b[c] = iJ[0] * Fx[c] + iJ[1] * Fy[c];
-      b[NP * NS + c] = iJ[2] * Fx[c] + iJ[3] * Fy[c];
-    }
+    put(b, up * BSTR, br);
+    put(b + NP * NS, up * BSTR, bs);
   }
-  for (int idx = tid; idx < ne_here * 3 * NFP; idx += NT) {
-    const int el = idx / (3 * NFP), fm = idx - el * 3 * NFP;
-    const int lf = fm / NFP, m = fm - lf * NFP, t = el & 1, cl = el >> 1;
-    const int cell = cell0 + cl;
-    const int cj = cell / args.nx, ci = cell - cj * args.nx;
-    const int ax = tab->axis[t][lf], dir = tab->dir[t][lf];
-    int code;
-    const int mode = face_mode(ax, dir, ax == 0 ? ci : cj, ax == 0 ? args.nx : args.ny, args.bc, code);
-    R qo[NC];
-    load_node<NC>(&q[(el * NP + tab->own_node[lf][m]) * NC], qo);
-    R nx = tab->normal[t][lf][0], ny = tab->normal[t][lf][1];
-    R scale = tab->fscale[t][lf];
-    // one face-flux call per face node (the 2D face functions build the
-    // BC ghost state themselves from the left state and the BC code)
-    R qn[NC];
-    if (mode == FACE_INTERIOR || mode == FACE_MIXED) {
-      const int nbt = tab->nb_t[t][lf], nbn = tab->nb_node[t][lf][m];
-      if (ax < 0) {
-        load_node<NC>(&q[((cl * 2 + nbt) * NP + nbn) * NC], qn);
-      } else {
-        const int ni = wrapi(ci + tab->off[t][lf][0], args.nx), nj = wrapi(cj + tab->off[t][lf][1], args.ny);
-        const R* gq = args.q_in + ((size_t(nj) * args.nx + ni) * 2 * NP + size_t(nbt) * NP + nbn) * NC;
+  __syncthreads();
+  for (int idx = tid; idx < npair * 5 * NFP; idx += NT) {
+    const int rest = idx / NFP, m = idx - rest * NFP, pr = rest / 5, wk = rest - pr * 5, cl = pr * LN;
+    const int up = cl + 1 < nc_here ? 1 : 0;
+    const int bits = tab->fbits[wk], nm = tab->fnode[wk][m];
+    const int t = bits & 1, lf = (bits >> 1) & 3, nbt = (bits >> 3) & 1, dd = (bits >> 6) & 3;
+    const bool own_left = bits & 0x100, diag = bits & 0x200;
+    const R *pl[LN], *pr_[LN];
+    int md[LN], any = 0;
 #pragma unroll
-        for (int c = 0; c < NC; ++c) qn[c] = __ldg(gq + c);
+    for (int k = 0; k < LN; ++k) {
+      const int c = cl + k * up;
+      const int2 cd = diag ? make_int2(0, 0) : sCd[c * 4 + dd];
+      md[k] = cd.y;
+      any |= cd.y;
+      const R* po = &q[((c * 2 + t) * NP + (nm & 255)) * NC];
+      const int nb = (nbt * NP + ((nm >> 8) & 255)) * NC;
+      const R* pn = diag ? q + c * 2 * NP * NC + nb : args.q_in + size_t(cd.x) * 2 * NP * NC + nb;
+      pl[k] = own_left ? po : pn;
+      pr_[k] = own_left ? pn : po;
+    }
+    T L[NC], Rr[NC], f[NC], nx = V::dup(tab->normal[t][lf][0]), ny = V::dup(tab->normal[t][lf][1]),
+                        s1 = V::dup(tab->fscale[t][lf]);
+    load(pl, L);
+    load(pr_, Rr);
+    if (any & 0xff) {
+      // boundary faces: the flux of (state, its ghost) -- the own trace, or
+      // with FACE_MIXED the neighbour's; a one-sided low face is its
+      // triangle's side 0, so normal and scale flip
+      R l[NC][LN], r[NC][LN], n[2][LN], sc[LN];
+      V::split(nx, n[0]);
+      V::split(ny, n[1]);
+      V::split(s1, sc);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        V::split(L[c], l[c]);
+        V::split(Rr[c], r[c]);
       }
-    } else {
 #pragma unroll
-      for (int c = 0; c < NC; ++c) qn[c] = qo[c];
-    }
-    if (mode == FACE_BC_LO) {
-      nx = -nx;
-      ny = -ny;
-      scale = -scale;
-    }
-    const bool bcf = mode != FACE_INTERIOR;
-    const bool own_left = tab->side[t][lf] == 0;
-    // left/right states by value (selecting between pointers would force
-    // the register arrays into local memory)
-    R L[NC], Rr[NC];
+      for (int k = 0; k < LN; ++k) {
+        const int mode = md[k] & 0xff;
+        if (mode == FACE_INTERIOR) continue;
+        const bool from_l = (mode == FACE_MIXED) != own_left;
+        R s[NC], g[NC];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      const R o = qo[c];
-      L[c] = bcf ? qn[c] : (own_left ? o : qn[c]);
-      Rr[c] = bcf ? qn[c] : (own_left ? qn[c] : o);
-    }
-    R f[NC];
-    ph.face(L, Rr, bcf ? code : int(BC_INTERIOR), nx, ny, f);
-    R* b = &sB[el * BSTR + (2 * NP + fm) * NS];
+        for (int c = 0; c < NC; ++c) s[c] = from_l ? l[c][k] : r[c][k];
+        if (mode == FACE_BC_LO) {
+          n[0][k] = -n[0][k];
+          n[1][k] = -n[1][k];
+          sc[k] = -sc[k];
+        }
+        ph.ghost(s, md[k] >> 8, n[0][k], n[1][k], g);
 #pragma unroll
-    for (int c = 0; c < NC; ++c) b[c] = scale * f[c];
+        for (int c = 0; c < NC; ++c) {
+          l[c][k] = s[c];
+          r[c][k] = g[c];
+        }
+      }
+      nx = V::make(n[0]);
+      ny = V::make(n[1]);
+      s1 = V::make(sc);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        L[c] = V::make(l[c]);
+        Rr[c] = V::make(r[c]);
+      }
+    }
+    P2::face(ph, L, Rr, nx, ny, f);
+    T v[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) v[c] = s1 * f[c];
+    put(&sB[(cl * 2 + t) * BSTR + (2 * NP + lf * NFP + m) * NS], up * 2 * BSTR, v);
+    if (diag) {  // the other triangle's row: same flux, its own scale
+      const int lf2 = (bits >> 4) & 3;
+      const T s2 = V::dup(tab->fscale[nbt][lf2]);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) v[c] = s2 * f[c];
+      put(&sB[(cl * 2 + nbt) * BSTR + (2 * NP + lf2 * NFP + (nm >> 16)) * NS], up * 2 * BSTR, v);
+    }
   }
   __syncthreads();
   const bool a_in = args.q_a == args.q_in, b_in = args.q_b == args.q_in;
@@ -186,6 +261,7 @@ __global__ void __launch_bounds__(NT) stage2d_kernel(Stage2DArgs<R> args, KuhnTa
   R* sQ = reinterpret_cast<R*>(smem_raw + 16 + kTabBytes);  // [2][QV]
   R* sB = sQ + 2 * QV;                                      // [EB][BSTR]
   R* sA = sB + EB * BSTR;                                   // [K][NP]
+  int2* sCd = reinterpret_cast<int2*>(sA + (K * NP + 1) / 2 * 2);  // [EC][4]
   const int tid = threadIdx.x;
   const int ngroups = (args.ncell + EC - 1) / EC;
   if (tid == 0) {
@@ -235,7 +311,7 @@ __global__ void __launch_bounds__(NT) stage2d_kernel(Stage2DArgs<R> args, KuhnTa
       for (int idx = tid; idx < ne_here * NP * NC; idx += NT) q[idx] = src[idx];
       __syncthreads();
     }
-    stage2d_tile<R, Phys, P, NT>(args, tab, ph, q, sB, sA, cell0, ne_here);
+    stage2d_tile<R, Phys, P, NT>(args, tab, ph, q, sB, sA, sCd, cell0, ne_here);
   }
 }
 
@@ -243,11 +319,11 @@ template <class R, int P, int NC>
 struct Cfg2 {
   using S = Stage2DShape<P, NC, R>;
   static constexpr int NP = S::NP;
-  static constexpr size_t kFixed = 16 + (sizeof(KuhnTab2<R>) + 15) / 16 * 16 + sizeof(R) * S::K * S::NP;
+  static constexpr size_t kFixed = 16 + (sizeof(KuhnTab2<R>) + 15) / 16 * 16 + sizeof(R) * (S::K * S::NP + 1);
   static constexpr int EC_RAW = int((100 * 1024 - kFixed) / S::kPerCell);
   static constexpr int EC = EC_RAW > 64 ? 64 : (EC_RAW < 1 ? 1 : EC_RAW);
   static constexpr int NT = 256;
-  static constexpr size_t kSmem = kFixed + sizeof(R) * (2 * size_t(2 * EC) * S::NP * NC + size_t(2 * EC) * S::BSTR);
+  static constexpr size_t kSmem = kFixed + sizeof(R) * (2 * size_t(2 * EC) * S::NP * NC + size_t(2 * EC) * S::BSTR) + EC * 32;
 };
 
 template <class R, class Phys, int P>

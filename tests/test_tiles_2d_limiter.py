@@ -1,0 +1,101 @@
+"""The 2D stage at the edges of its tiles, and the limiter at the edges of its
+chunks.
+
+The 2D stage takes cells in pairs (FP32) inside tiles of up to 64 cells;
+odd cell counts leave a pair with one cell, 65 and 129 cells a tile of one.
+The limiter works in chunks of 128 elements: meshes on both sides of one and
+two chunks, with every boundary kind.  Right-hand sides and limited states are
+compared with the FP64 oracle; bounds: FP32 arithmetic over K <= 60 columns of
+O(1) operands, 4e-6 as for the oracle's own FP32 path, FP64 the oracle's
+operator construction (tests/dgcases.py); the limiter's arithmetic is a few
+operations on states of O(1): 4 ulp."""
+import numpy as np
+import pytest
+
+import mojoxm_b200 as M
+from tests import dgcases as C
+
+CELLS = [(1, 1), (3, 1), (1, 5), (7, 3), (13, 5), (43, 3)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("name,P", [("euler_hlle", 1), ("euler_hlle", 4), ("euler_rusanov", 2), ("euler_hllc", 3),
+                                    ("shallow_water", 5), ("shallow_water_hll", 2), ("maxwell", 3), ("advection", 2),
+                                    ("mhd_glm", 2), ("mhd_plain", 3)])
+@pytest.mark.parametrize("bcs", ["periodic", "inflow_outflow", "mixed_hi_only"])
+def test_rhs_on_partial_tiles_2d(oracle_mod, name, P, prec, bcs):
+    ph, L = C.PHYSICS_2D[name](), (1.0, 0.8)
+    for n in CELLS:
+        s = M.Solver(M.Mesh(*n, 1, *L, 1.0, bcs=M.BoundaryConditions(*C.BCS_2D[bcs], 0, 0), dim=2), ph, P=P,
+                     precision=prec)
+        o = oracle_mod.Oracle2D(P, n, L, M.physics_dict(ph), C.BCS_2D[bcs])
+        q = C.random_state(s.shape, ph, seed=sum(n)).astype(np.float32).astype(np.float64)
+        err = C.rel_err(s.rhs(q), o.rhs(q))
+        s.close()
+        assert err < (4e-6 if prec == "f32" else C.TOL_F64_2D[P]), (n, err)
+
+
+@pytest.mark.gpu
+def test_hlle_entropy_fix_2d(oracle_mod):
+    """The out-of-line branch of the packed HLLE flux."""
+    ph, n = C.euler(M.FLUX_HLLE, efix=True), (7, 5)
+    for prec, tol in (("f32", 4e-6), ("f64", 1e-11)):
+        s = M.Solver(M.Mesh(*n, 1, 1.0, 0.8, 1.0, dim=2), ph, P=3, precision=prec)
+        o = oracle_mod.Oracle2D(3, n, (1.0, 0.8), M.physics_dict(ph))
+        q = C.random_state(s.shape, ph, seed=5).astype(np.float32).astype(np.float64)
+        err = C.rel_err(s.rhs(q), o.rhs(q))
+        s.close()
+        assert err < tol, (prec, err)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim,n", [(3, (1, 1, 1)), (3, (7, 3, 1)), (3, (3, 2, 4)), (3, (5, 3, 3)), (2, (1, 1)),
+                                   (2, (8, 8)), (2, (13, 5)), (2, (16, 9))])
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+def test_limiter_on_chunk_edges(oracle_mod, dim, n, prec):
+    ph = C.euler(M.FLUX_HLLE)
+    for name in ("periodic", "inflow_outflow"):
+        b3, b2 = C.BCS_3D[name], C.BCS_2D[name]
+        if dim == 3:
+            mesh = M.Mesh(*n, bcs=M.BoundaryConditions(*b3))
+            o = oracle_mod.Oracle3D(2, n, 1.0, M.physics_dict(ph), b3)
+        else:
+            mesh = M.Mesh(*n, 1, bcs=M.BoundaryConditions(*b2, 0, 0), dim=2)
+            o = oracle_mod.Oracle2D(2, n, 1.0, M.physics_dict(ph), b2)
+        s = M.Solver(mesh, ph, P=2, precision=prec)
+        s.enable_cell_limiter(True, 0.1)
+        o.enable_limiter(True, 0.1)
+        q = C.random_state(s.shape, ph, seed=9).astype(np.float32).astype(np.float64)
+        s.upload_state(q)
+        o.set(q)
+        s.limit()
+        o.limit()
+        a, b = s.download_state().astype(np.float64), o.get()
+        s.close()
+        assert C.rel_err(a, q) > 1e-3  # the random states are limited
+        assert C.rel_err(a, b) < (1e-6 if prec == "f32" else 1e-14), C.rel_err(a, b)
+
+
+@pytest.mark.gpu
+def test_reductions_return_to_zero_state(oracle_mod):
+    """Maxima and sums of different grids in turn on one handle, and more
+    handles than there are host result words: every call starts from the
+    state the previous one left."""
+    ph = C.euler(M.FLUX_RUSANOV)
+    many = [M.Solver(M.Mesh(3, 2, 1, dim=2), ph, P=1) for _ in range(260)]
+    big = M.Solver(M.Mesh(40, 30, 1, dim=2), ph, P=2)
+    for s in (many[0], many[-1], big):
+        q = C.random_state(s.shape, ph, seed=4)
+        s.upload_state(q)
+        u = np.hypot(q[..., 1], q[..., 2]) / q[..., 0]
+        p = 0.4 * (q[..., 3] - 0.5 * q[..., 0] * u * u)
+        lam = float((u + np.sqrt(1.4 * p / q[..., 0])).max())
+        for _ in range(3):
+            assert abs(s.max_wavespeed() - lam) < 1e-13 * lam
+            assert abs(s.integral(0, kind=2) - q[..., 0].max()) < 1e-15
+            assert abs(s.integral(3, kind=3) - q[..., 3].mean()) < 1e-13 * q[..., 3].mean()
+        s.upload_state(0.25 * q)  # a smaller maximum after a larger one
+        assert abs(s.integral(0, kind=2) - 0.25 * q[..., 0].max()) < 1e-15
+    for s in many + [big]:
+        s.close()
