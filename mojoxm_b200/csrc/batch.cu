@@ -88,7 +88,7 @@ struct Batch {
 
 namespace {
 
-constexpr int kLimChunk = 128;      // elements per limiter block
+constexpr int kLimChunk = kLimBlock;  // elements per limiter block
 constexpr size_t kSmemCap = 200 * 1024;
 const int kEcCandidates[] = {1, 2, 4, 8, 16, 32, 64};
 
@@ -172,7 +172,7 @@ template <class R, int NC>
 cudaError_t lim3_launch_nc(const Lim3Group& lg, int which, cudaStream_t st) {
   const LimBatch3<R> lb{(const LimDesc3<R>*)lg.d_desc, lg.d_items, lg.nitems, which};
   avg3d_batch_kernel<R, NC><<<lg.nitems, 256, 0, st>>>(lb);
-  theta3d_batch_kernel<R, NC><<<lg.nitems, 32 * kLim3Epb, 0, st>>>(lb);
+  theta3d_batch_kernel<R, NC><<<lg.nitems, kLimBlock, 0, st>>>(lb);
   return cudaGetLastError();
 }
 
@@ -471,8 +471,6 @@ void build(Batch* b) {
     CK(cudaMalloc(&g.d_counter, 3 * sizeof(int)));
     g.grid = grid_for<R>(b, g, g.smem, g.nitems);
   }
-  for (auto& g : b->groups)
-    if (g.dim == 2 && g.nlitems > 0) CK(prepare_lim2d_batch<R>(g.NC));
   build_lim3<R>(b);
   // first-use set-up of the batched 3D kernels (kernel attributes,
   // occupancy) before the capture: an empty batch launches nothing

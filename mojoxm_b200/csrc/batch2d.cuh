@@ -228,23 +228,24 @@ __global__ void avg_batch_kernel(LimBatch2DArgs<R> la) {
   }
 }
 
-// Theta + apply of one chunk (blocks of kLim2dBlock threads, chunks of at
-// most kLim2dBlock elements): the single-solve limiter's staged block
-// function on this solve's buffers and table.  Dynamic shared memory sized
-// for P = 5.
+// Theta + apply of one chunk: the single-solve limiter's block function on
+// this solve's buffers and table.
 template <class R, int NC>
-__global__ void __launch_bounds__(kLim2dBlock) theta_batch_kernel(LimBatch2DArgs<R> la) {
-  extern __shared__ __align__(16) unsigned char lim_smem[];
+__global__ void __launch_bounds__(kLimBlock) theta_batch_kernel(LimBatch2DArgs<R> la) {
+  __shared__ LimShared<R> sh;
   const int4 item = la.items[blockIdx.x];
   const SolveDesc2<R>* sd = &la.solves[item.x];
   R* q = sd->q[la.which];
-  const R* ext = sd->avg + int64_t(2) * sd->ncell * NC;
+  auto run = [&](auto np) {
+    theta_block<R, 2, decltype(np)::value, NC>(q, sd->avg, sd->avg + int64_t(2) * sd->ncell * NC, item.y, item.z,
+                                               sd->tab, sd->nx, sd->ny, 1, sd->bc, sd->eps2, sh);
+  };
   switch (item.w) {
-    case 1: theta2d_block<R, ntri(1), NC>(q, sd->avg, ext, item.y, item.z, sd->tab, sd->nx, sd->ny, sd->bc, sd->eps2, lim_smem); break;
-    case 2: theta2d_block<R, ntri(2), NC>(q, sd->avg, ext, item.y, item.z, sd->tab, sd->nx, sd->ny, sd->bc, sd->eps2, lim_smem); break;
-    case 3: theta2d_block<R, ntri(3), NC>(q, sd->avg, ext, item.y, item.z, sd->tab, sd->nx, sd->ny, sd->bc, sd->eps2, lim_smem); break;
-    case 4: theta2d_block<R, ntri(4), NC>(q, sd->avg, ext, item.y, item.z, sd->tab, sd->nx, sd->ny, sd->bc, sd->eps2, lim_smem); break;
-    default: theta2d_block<R, ntri(5), NC>(q, sd->avg, ext, item.y, item.z, sd->tab, sd->nx, sd->ny, sd->bc, sd->eps2, lim_smem); break;
+    case 1: run(std::integral_constant<int, ntri(1)>{}); break;
+    case 2: run(std::integral_constant<int, ntri(2)>{}); break;
+    case 3: run(std::integral_constant<int, ntri(3)>{}); break;
+    case 4: run(std::integral_constant<int, ntri(4)>{}); break;
+    default: run(std::integral_constant<int, ntri(5)>{}); break;
   }
 }
 

@@ -81,29 +81,9 @@ cudaError_t launch_stage2d_batch(const mxm_dg_physics_desc& pd, const Batch2DArg
 }
 
 template <class R, int NC>
-cudaError_t lim2d_batch_attr() {
-  return cudaFuncSetAttribute(theta_batch_kernel<R, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              int(lim2d_smem_bytes<R, ntri(5), NC>()));
-}
-
-// Kernel attributes of the batched limiter (call before any stream capture).
-template <class R>
-cudaError_t prepare_lim2d_batch(int NC) {
-  switch (NC) {
-    case 1: return lim2d_batch_attr<R, 1>();
-    case 3: return lim2d_batch_attr<R, 3>();
-    case 4: return lim2d_batch_attr<R, 4>();
-    case 6: return lim2d_batch_attr<R, 6>();
-    case 7: return lim2d_batch_attr<R, 7>();
-  }
-  return cudaErrorInvalidValue;
-}
-
-template <class R, int NC>
 cudaError_t lim2d_batch_nc(const LimBatch2DArgs<R>& la, cudaStream_t st) {
-  constexpr size_t smem = lim2d_smem_bytes<R, ntri(5), NC>();
   avg_batch_kernel<R, NC><<<la.nitems, 256, 0, st>>>(la);
-  theta_batch_kernel<R, NC><<<la.nitems, kLim2dBlock, smem, st>>>(la);
+  theta_batch_kernel<R, NC><<<la.nitems, kLimBlock, 0, st>>>(la);
   return cudaGetLastError();
 }
 
@@ -124,7 +104,6 @@ cudaError_t launch_lim2d_batch(int NC, const LimBatch2DArgs<R>& la, cudaStream_t
   template cudaError_t stage2d_batch_blocks_per_sm<R>(const mxm_dg_physics_desc&, size_t, int*);                   \
   template cudaError_t launch_stage2d_batch<R>(const mxm_dg_physics_desc&, const Batch2DArgs<R>&, int, size_t,     \
                                                cudaStream_t);                                                       \
-  template cudaError_t launch_lim2d_batch<R>(int, const LimBatch2DArgs<R>&, cudaStream_t);                       \
-  template cudaError_t prepare_lim2d_batch<R>(int);
+  template cudaError_t launch_lim2d_batch<R>(int, const LimBatch2DArgs<R>&, cudaStream_t);
 
 }  // namespace mxm

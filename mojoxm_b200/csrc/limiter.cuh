@@ -13,8 +13,7 @@
 // enters theta the least and the largest of its nodal values; pass 2 gets
 // theta from those extrema and the neighbours' means without reading the
 // nodal state, and reads and rewrites the values of the elements with
-// theta < 1 only (3D: a warp per element; 2D: a block per chunk of
-// elements, theta2d_block).
+// theta < 1 only (a block per chunk of elements, theta_block).
 //
 // Why the extrema suffice: the ratio alpha(d) = (D^2 + 2 D d + eps^2) /
 // (D^2 + 2 d^2 + D d + eps^2) of a node with deviation magnitude d from the
@@ -33,22 +32,11 @@
 // {least, largest} nodal value of component c of element e, for the NCT
 // components that enter theta (every component in 3D, component 0 in 2D).
 #pragma once
+#include <type_traits>
+
 #include "dg_common.cuh"
 
 namespace mxm {
-
-template <class R, int NP, int NC>
-__global__ void cell_avg_kernel(LimArgs<R> a) {
-  const int64_t tid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (tid >= a.ne * NC) return;
-  const int64_t e = tid / NC;
-  const int c = int(tid - e * NC);
-  const R* q = a.q + e * NP * NC + c;
-  R s = R(0);
-#pragma unroll
-  for (int n = 0; n < NP; ++n) s = fma(__ldg(&a.w[n]), q[n * NC], s);
-  a.avg[tid] = s;
-}
 
 template <class R, int NP, int NC, int NCT>
 __global__ void cell_avg_kernel(LimArgs<R> a) {
@@ -100,86 +88,118 @@ __device__ __forceinline__ R theta_from_extrema(R own, R lo, R hi, R umin, R uma
   return th;
 }
 
-// Theta + apply of element e (< a.e1) by one warp; every lane of the warp
-// calls it with the same e.
-template <class R, int DIM, int NP, int NC>
-__device__ __forceinline__ void theta_apply_elem(const LimArgs<R>& a, const KuhnTab3<R>& t3, const KuhnTab2<R>& t2,
-                                                 int64_t e) {
-  constexpr int NTYPE = DIM == 3 ? 6 : 2, NFACE = DIM + 1, VALS = NP * NC;
+// Theta + apply of up to kLimBlock consecutive elements by a block of
+// kLimBlock threads.
+//  (1) One thread per element resolves its neighbours and gets theta from
+//      the means and the element's nodal extrema; the limited elements are
+//      listed in shared memory.
+//  (2) One thread per value rewrites the listed elements, over consecutive
+//      values.
+// What bounds it is the latency of (1)'s dependent loads: the face treatment
+// is packed into one word per (type, face) in shared memory first (a
+// per-lane index into the parameter bank costs one access per distinct
+// word), and the cell position takes no integer division.  A warp per
+// element with a lane per component and a lane per face, as this pass was
+// before, kept 27 of 32 lanes idle.  Means and theta pass together: 449 ->
+// 262 us on 663,552 P5 tets of five components (142 of it the means), 51 ->
+// 27 us on 82,944 P3 tets, 16.6 -> 12.5 us on 20,000 P2 triangles.
+// Faces whose neighbour is the element itself (boundary faces) do not
+// constrain.  `ext` holds the extrema of the components that enter theta.
+constexpr int kLimBlock = 128;
+template <class R>
+struct LimShared {
+  int face[24];  // (axis + 1) | (dir > 0) << 2 | nb_t << 3, index t * faces + lf
+  int count, list[kLimBlock];
+  R th[kLimBlock];
+};
+
+template <class R, int DIM, int NP, int NC, class Tab>
+__device__ __forceinline__ void theta_block(R* q, const R* avg, const R* ext, int64_t e0, int ne, const Tab& tab, int nx,
+                                            int ny, int nz, const int* bc, R eps2, LimShared<R>& sh) {
+  constexpr int NTYPE = DIM == 3 ? 6 : 2, NF = DIM + 1, VALS = NP * NC;
   constexpr int NCT = DIM == 3 ? NC : 1;  // components entering theta
-  const int lane = threadIdx.x & 31;
-  const int t = int(e % NTYPE);
-  const int64_t cell = e / NTYPE;
-  int cpos[3];
-  if (DIM == 3) {
-    const int64_t nxy = int64_t(a.nx) * a.ny;
-    cpos[2] = int(cell / nxy);
-    const int64_t rem = cell - int64_t(cpos[2]) * nxy;
-    cpos[1] = int(rem / a.nx);
-    cpos[0] = int(rem - int64_t(cpos[1]) * a.nx);
-  } else {
-    cpos[1] = int(cell / a.nx);
-    cpos[0] = int(cell - int64_t(cpos[1]) * a.nx);
-    cpos[2] = 0;
+  const int tid = threadIdx.x;
+  if (tid < NTYPE * NF) {
+    const int t = tid / NF, lf = tid - t * NF;
+    sh.face[tid] = (tab.axis[t][lf] + 1) | (tab.dir[t][lf] > 0 ? 4 : 0) | (tab.nb_t[t][lf] << 3);
   }
-  const int ncells[3] = {a.nx, a.ny, a.nz};
-  // neighbour elements: lanes 0..NFACE-1 each resolve one face
-  int64_t nb = e;
-  if (lane < NFACE) {
-    const int lf = lane;
-    const int ax = DIM == 3 ? t3.axis[t][lf] : t2.axis[t][lf];
-    const int dir = DIM == 3 ? t3.dir[t][lf] : t2.dir[t][lf];
-    int code;
-    const int mode = face_mode(ax, dir, ax >= 0 ? cpos[ax] : 0, ax >= 0 ? ncells[ax] : 1, a.bc, code);
-    if (mode == FACE_INTERIOR || mode == FACE_MIXED) {
-      if (DIM == 3) {
-        const int ni = wrapi(cpos[0] + t3.off[t][lf][0], a.nx), nj = wrapi(cpos[1] + t3.off[t][lf][1], a.ny),
-                  nk = wrapi(cpos[2] + t3.off[t][lf][2], a.nz);
-        nb = (int64_t(ni) + int64_t(a.nx) * (nj + int64_t(a.ny) * nk)) * 6 + t3.nb_t[t][lf];
-      } else {
-        const int ni = wrapi(cpos[0] + t2.off[t][lf][0], a.nx), nj = wrapi(cpos[1] + t2.off[t][lf][1], a.ny);
-        nb = (int64_t(nj) * a.nx + ni) * 2 + t2.nb_t[t][lf];
+  if (tid == kLimBlock - 1) sh.count = 0;
+  __syncthreads();
+  if (tid < ne) {
+    const int e = int(e0) + tid, cell = e / NTYPE, t = e - cell * NTYPE;
+    int pos[3] = {cell, 0, 0};
+    if (DIM == 3) {
+      pos[2] = div_cells(cell, nx * ny);
+      pos[0] -= pos[2] * nx * ny;
+    }
+    pos[1] = div_cells(pos[0], nx);
+    pos[0] -= pos[1] * nx;
+    int nb[NF];
+#pragma unroll
+    for (int lf = 0; lf < NF; ++lf) {
+      const int f = sh.face[t * NF + lf], ax = (f & 3) - 1, dir = f & 4 ? 1 : -1;
+      const int n = ax == 0 ? nx : (ax == 1 ? ny : nz), p = ax == 0 ? pos[0] : (ax == 1 ? pos[1] : pos[2]);
+      int code;
+      const int mode = face_mode(ax, dir, p, n, bc, code);
+      nb[lf] = e;
+      if (mode == FACE_INTERIOR || mode == FACE_MIXED) {
+        const int step = ax < 0 ? 0 : (wrapi(p + dir, n) - p) * (ax == 0 ? 1 : (ax == 1 ? nx : nx * ny));
+        nb[lf] = (cell + step) * NTYPE + (f >> 3);
       }
     }
-  }
-  int64_t nbs[NFACE];
+    R th = R(1);
 #pragma unroll
-  for (int lf = 0; lf < NFACE; ++lf) nbs[lf] = __shfl_sync(0xffffffffu, nb, lf);
-  // lane c < NCT: theta of component c
-  R th = R(1);
-  if (lane < NCT) {
-    const int c = lane;
-    const R own = a.avg[e * NC + c];
-    R lo = own, hi = own;
+    for (int c = 0; c < NCT; ++c) {
+      const R own = avg[size_t(e) * NC + c];
+      R lo = own, hi = own;
 #pragma unroll
-    for (int lf = 0; lf < NFACE; ++lf) {
-      if (DIM == 2 && nbs[lf] == e) continue;  // 2D: BC faces do not constrain
-      const R v = a.avg[nbs[lf] * NC + c];
-      if (v < lo) lo = v;
-      if (v > hi) hi = v;
+      for (int lf = 0; lf < NF; ++lf) {
+        const R v = avg[size_t(nb[lf]) * NC + c];
+        if (v < lo) lo = v;
+        if (v > hi) hi = v;
+      }
+      const R* x = ext + (size_t(e) * NCT + c) * 2;
+      const R tc = theta_from_extrema(own, lo, hi, x[0], x[1], eps2);
+      th = tc < th ? tc : th;
     }
-    const R* x = a.avg + a.ne * NC + (e * NCT + c) * 2;
-    th = theta_from_extrema(own, lo, hi, x[0], x[1], a.eps2);
+    if (th < R(1)) {
+      const int k = atomicAdd(&sh.count, 1);
+      sh.list[k] = tid;
+      sh.th[k] = th;
+    }
   }
+  __syncthreads();
+  // eight values a thread in flight: the loads of a batch come before its
+  // stores (the compiler may not move a load over a store that could alias)
+  const int n = sh.count * VALS;
+  constexpr int U = 8;
+  for (int i0 = tid; i0 < n; i0 += U * kLimBlock) {
+    R x[U], bm[U], th[U];
+    size_t at[U];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const R v = __shfl_xor_sync(0xffffffffu, th, o);
-    th = v < th ? v : th;
-  }
-  if (!(th < R(1))) return;
-  R* qe = a.q + e * VALS;
-  for (int idx = lane; idx < VALS; idx += 32) {
-    const int c = idx % NC;
-    const R bm = a.avg[e * NC + c];
-    qe[idx] = bm + th * (qe[idx] - bm);
+    for (int u = 0; u < U; ++u) {
+      const int idx = min(i0 + u * kLimBlock, n - 1), k = idx / VALS, v = idx - k * VALS;
+      const size_t e = size_t(e0) + sh.list[k];
+      at[u] = e * VALS + v;
+      x[u] = q[at[u]];
+      bm[u] = avg[e * NC + v % NC];
+      th[u] = sh.th[k];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i0 + u * kLimBlock < n) q[at[u]] = bm[u] + th[u] * (x[u] - bm[u]);
   }
 }
 
-// One warp per element; EPB elements per block of 32*EPB threads.
-template <class R, int DIM, int NP, int NC, int EPB>
-__global__ void __launch_bounds__(32 * EPB) theta_apply_kernel(LimArgs<R> a, KuhnTab3<R> t3, KuhnTab2<R> t2) {
-  const int64_t e = a.e0 + int64_t(blockIdx.x) * EPB + (threadIdx.x >> 5);
-  if (e < a.e1) theta_apply_elem<R, DIM, NP, NC>(a, t3, t2, e);
+template <class R, int DIM, int NP, int NC>
+__global__ void __launch_bounds__(kLimBlock) theta_kernel(LimArgs<R> a, const __grid_constant__ KuhnTab3<R> t3,
+                                                          const __grid_constant__ KuhnTab2<R> t2) {
+  __shared__ LimShared<R> sh;
+  const int64_t e0 = a.e0 + int64_t(blockIdx.x) * kLimBlock;
+  const int ne = int(a.e1 - e0 < kLimBlock ? a.e1 - e0 : kLimBlock);
+  const R* ext = a.avg + a.ne * NC;
+  if constexpr (DIM == 3) theta_block<R, 3, NP, NC>(a.q, a.avg, ext, e0, ne, t3, a.nx, a.ny, a.nz, a.bc, a.eps2, sh);
+  else theta_block<R, 2, NP, NC>(a.q, a.avg, ext, e0, ne, t2, a.nx, a.ny, 1, a.bc, a.eps2, sh);
 }
 
 // ---- batched 3D limiter: the cell-mean and theta passes of many limited
@@ -197,7 +217,7 @@ struct LimBatch3 {
   const int4* items;  // {solve, first element, elements, 0}
   int nitems, which;
 };
-constexpr int kLim3Chunk = 128, kLim3Epb = 8;
+constexpr int kLim3Chunk = kLimBlock;
 
 template <class R, int NP, int NC>
 __device__ __forceinline__ void avg3d_chunk(const LimDesc3<R>& d, R* q, int64_t e0, int ne) {
@@ -234,97 +254,23 @@ __global__ void avg3d_batch_kernel(LimBatch3<R> lb) {
   }
 }
 
-// The elements of a chunk, one warp each in turn.
-template <class R, int NP, int NC>
-__device__ __forceinline__ void theta3d_chunk(const LimDesc3<R>& d, R* q, int64_t e0, int ne) {
-  LimArgs<R> a = d.a;
-  a.q = q;
-  a.e1 = e0 + ne;
-  for (int g = threadIdx.x >> 5; g < ne; g += kLim3Epb) theta_apply_elem<R, 3, NP, NC>(a, d.tab, KuhnTab2<R>{}, e0 + g);
-}
-
 template <class R, int NC>
-__global__ void __launch_bounds__(32 * kLim3Epb) theta3d_batch_kernel(LimBatch3<R> lb) {
+__global__ void __launch_bounds__(kLimBlock) theta3d_batch_kernel(LimBatch3<R> lb) {
+  __shared__ LimShared<R> sh;
   const int4 it = lb.items[blockIdx.x];
   const LimDesc3<R>& d = lb.solves[it.x];
   R* q = d.qs[lb.which];
+  auto run = [&](auto np) {
+    theta_block<R, 3, decltype(np)::value, NC>(q, d.a.avg, d.a.avg + d.a.ne * NC, it.y, it.z, d.tab, d.a.nx, d.a.ny,
+                                               d.a.nz, d.a.bc, d.a.eps2, sh);
+  };
   switch (d.P) {
-    case 1: theta3d_chunk<R, ntet(1), NC>(d, q, it.y, it.z); break;
-    case 2: theta3d_chunk<R, ntet(2), NC>(d, q, it.y, it.z); break;
-    case 3: theta3d_chunk<R, ntet(3), NC>(d, q, it.y, it.z); break;
-    case 4: theta3d_chunk<R, ntet(4), NC>(d, q, it.y, it.z); break;
-    default: theta3d_chunk<R, ntet(5), NC>(d, q, it.y, it.z); break;
+    case 1: run(std::integral_constant<int, ntet(1)>{}); break;
+    case 2: run(std::integral_constant<int, ntet(2)>{}); break;
+    case 3: run(std::integral_constant<int, ntet(3)>{}); break;
+    case 4: run(std::integral_constant<int, ntet(4)>{}); break;
+    default: run(std::integral_constant<int, ntet(5)>{}); break;
   }
-}
-
-// A block of kLim2dBlock threads limits up to kLim2dBlock consecutive
-// elements: (1) one thread per element resolves its cell mean and the
-// neighbours' bounds (component 0; BC faces skipped) and gets theta from
-// the element's nodal extrema of component 0 (theta_from_extrema); (2) one
-// thread per value rewrites the values of the elements with theta < 1, over
-// consecutive values of the chunk.  The arithmetic is the reference's 2D
-// limiter (src/local_mesh_2d_gpu_limiter.mojo:74-153): theta from component
-// 0, faces whose neighbour resolves to the element itself (BC faces) do not
-// constrain, theta scales every component's deviation from its cell mean.
-// `ext` holds the extrema (one theta component).  Dynamic shared memory
-// lim2d_smem_bytes<R, NP, NC>().
-constexpr int kLim2dBlock = 128;
-template <class R, int NP, int NC>
-constexpr size_t lim2d_smem_bytes() {
-  return size_t(kLim2dBlock) * sizeof(R);
-}
-
-template <class R, int NP, int NC>
-__device__ __forceinline__ void theta2d_block(R* q, const R* avg, const R* ext, int64_t e0, int ne,
-                                              const KuhnTab2<R>& tab, int nx, int ny, const int* bc, R eps2,
-                                              unsigned char* smem) {
-  constexpr int VALS = NP * NC;
-  R* s_th = reinterpret_cast<R*>(smem);
-  const int tid = threadIdx.x;
-  bool lim = false;
-  if (tid < ne) {
-    const int64_t e = e0 + tid;
-    const int t = int(e & 1);
-    const int64_t cell = e >> 1;
-    const int cj = int(cell / nx), ci = int(cell - int64_t(cj) * nx);
-    const R own = avg[e * NC];
-    R lo = own, hi = own;
-#pragma unroll
-    for (int lf = 0; lf < 3; ++lf) {
-      const int ax = tab.axis[t][lf], dir = tab.dir[t][lf];
-      int code;
-      const int mode = face_mode(ax, dir, ax == 0 ? ci : cj, ax == 0 ? nx : ny, bc, code);
-      if (mode != FACE_INTERIOR && mode != FACE_MIXED) continue;
-      const int ni = wrapi(ci + tab.off[t][lf][0], nx), nj = wrapi(cj + tab.off[t][lf][1], ny);
-      const int64_t nb = (int64_t(nj) * nx + ni) * 2 + tab.nb_t[t][lf];
-      if (nb == e) continue;
-      const R v = avg[nb * NC];
-      if (v < lo) lo = v;
-      if (v > hi) hi = v;
-    }
-    const R th = theta_from_extrema(own, lo, hi, ext[e * 2], ext[e * 2 + 1], eps2);
-    s_th[tid] = th;
-    lim = th < R(1);
-  }
-  if (!__syncthreads_or(lim)) return;  // no element of the chunk is limited
-  R* base = q + e0 * VALS;
-#pragma unroll 4
-  for (int idx = tid; idx < ne * VALS; idx += blockDim.x) {
-    const int el = idx / VALS;
-    const R th = s_th[el];
-    if (!(th < R(1))) continue;
-    const int c = (idx - el * VALS) % NC;
-    const R bm = avg[(e0 + el) * NC + c];
-    base[idx] = bm + th * (base[idx] - bm);
-  }
-}
-
-template <class R, int NP, int NC>
-__global__ void __launch_bounds__(kLim2dBlock) theta2d_kernel(LimArgs<R> a, KuhnTab2<R> t2) {
-  extern __shared__ __align__(16) unsigned char lim_smem[];
-  const int64_t e0 = int64_t(blockIdx.x) * kLim2dBlock;
-  const int ne = int(a.ne - e0 < kLim2dBlock ? a.ne - e0 : kLim2dBlock);
-  theta2d_block<R, NP, NC>(a.q, a.avg, a.avg + a.ne * NC, e0, ne, t2, a.nx, a.ny, a.bc, a.eps2, lim_smem);
 }
 
 // ---- FP64 reductions: per-block partial sums, then a fixed-order final sum.
