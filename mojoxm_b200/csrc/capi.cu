@@ -423,7 +423,7 @@ cudaError_t stage_launch(Handle* h, const void* qi, const void* qa, const void* 
 }
 
 template <class R>
-cudaError_t wavespeed_launch(Handle* h, const void* qi, unsigned long long* out) {
+cudaError_t wavespeed_launch(Handle* h, const void* qi, const ReduceOut& out) {
   const double* p = h->phys.p;
   if (h->dim == 3) {
     Stage3DArgs<R> ar{};
@@ -669,6 +669,45 @@ void dev_free(Handle* h, void* p) {
   if (p) cudaFreeAsync(p, h->stream);
 }
 
+// Result words in host memory that the device writes: one page of the
+// process, a 64-byte slot per handle from its creation to its end (handles
+// beyond the page's slots, or without it, copy their results back).
+namespace {
+constexpr int kHostSlots = 256;
+std::mutex g_slot_mu;
+double* g_slots = nullptr;
+bool g_slots_tried = false, g_slot_used[kHostSlots] = {};
+}  // namespace
+
+double* host_slot_take() {
+  std::lock_guard<std::mutex> g(g_slot_mu);
+  if (!g_slots_tried) {
+    g_slots_tried = true;
+    if (cudaHostAlloc((void**)&g_slots, kHostSlots * 64, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+      cudaGetLastError();
+      g_slots = nullptr;
+    }
+  }
+  for (int k = 0; g_slots && k < kHostSlots; ++k)
+    if (!g_slot_used[k]) {
+      g_slot_used[k] = true;
+      return g_slots + k * 8;
+    }
+  return nullptr;
+}
+
+void host_slot_give(double* p) {
+  std::lock_guard<std::mutex> g(g_slot_mu);
+  if (p) g_slot_used[(p - g_slots) / 8] = false;
+}
+
+// The value a reduction on the handle's stream left in its result word.
+void fetch_result(Handle* h, double* out) {
+  if (!h->hres) CK(cudaMemcpyAsync(out, h->dscalar, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
+  if (h->hres) *out = *const_cast<volatile double*>(h->hres);
+}
+
 std::vector<float> xyz_f32(const Handle* h) {
   std::vector<float> x(size_t(h->ne) * h->NP * h->dim);
   if (h->dim == 3) {
@@ -772,6 +811,7 @@ void destroy(Handle* h) {
   if (!h) return;
   cudaSetDevice(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
+  host_slot_give(h->hres);
   for (void* p : {h->q[0], h->q[1], h->q[2], h->A, h->w, h->avg, static_cast<void*>(h->xyz),
                   static_cast<void*>(h->partial), static_cast<void*>(h->dscalar), static_cast<void*>(h->uscalar),
                   static_cast<void*>(h->derr), h->tcimg})
@@ -927,6 +967,8 @@ Handle* create(const mxm_dg_mesh_desc* m, const mxm_dg_physics_desc* ph, int P, 
     dev_alloc(raw, reinterpret_cast<void**>(&raw->uscalar), 4 * sizeof(unsigned long long));
     dev_alloc(raw, reinterpret_cast<void**>(&raw->derr), sizeof(int));
     CK(cudaMemsetAsync(raw->derr, 0, sizeof(int), raw->stream));
+    CK(cudaMemsetAsync(raw->uscalar, 0, 4 * sizeof(unsigned long long), raw->stream));
+    raw->hres = host_slot_take();
     CK(cudaStreamSynchronize(raw->stream));
   } catch (...) {
     h.release();
@@ -1212,14 +1254,10 @@ int mxm_dg_advance_host_async(void* handle, const void* q_host, void* q_out_host
 
 int mxm_dg_max_wavespeed(void* handle, double* out) {
   API_BEGIN
-  CK(cudaMemsetAsync(h->uscalar, 0, sizeof(unsigned long long), h->stream));
-  cudaError_t e = h->rbytes == 8 ? mxm::wavespeed_launch<double>(h, h->q[0], h->uscalar)
-                                 : mxm::wavespeed_launch<float>(h, h->q[0], h->uscalar);
+  const mxm::ReduceOut r{h->uscalar, (unsigned*)(h->uscalar + 1), h->hres ? h->hres : h->dscalar};
+  cudaError_t e = h->rbytes == 8 ? mxm::wavespeed_launch<double>(h, h->q[0], r) : mxm::wavespeed_launch<float>(h, h->q[0], r);
   if (e != cudaSuccess) throw mxm::CudaError(e, "wavespeed launch");
-  unsigned long long bits = 0;
-  CK(cudaMemcpyAsync(&bits, h->uscalar, sizeof(bits), cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
-  std::memcpy(out, &bits, sizeof(double));
+  mxm::fetch_result(h, out);
   if (!(*out < 1.0e300)) {
     h->err = "non-finite wave speed";
     return MXM_DG_ENONFINITE;
@@ -1233,16 +1271,16 @@ int mxm_dg_reduce_conserved(void* handle, int which, int c, int kind, double* ou
     throw mxm::ArgError("which 0..2, component in range, kind 0..4");
   const double scale = mxm::reduce_scale(h, kind);
   const size_t off = size_t(h->own_e0()) * h->NP * h->NC;  // owned elements only
+  double* res = h->hres ? h->hres : h->dscalar;
   cudaError_t e = h->rbytes == 8
                       ? mxm::launch_reduce<double>(h->P, h->dim, h->NC, (const double*)h->q[which] + off,
                                                    (const double*)h->w, h->own_ne(), c, kind, scale, h->partial,
-                                                   h->npartial, h->dscalar, h->stream)
+                                                   h->npartial, (unsigned*)(h->uscalar + 1), res, h->stream)
                       : mxm::launch_reduce<float>(h->P, h->dim, h->NC, (const float*)h->q[which] + off,
                                                   (const float*)h->w, h->own_ne(), c, kind, scale, h->partial,
-                                                  h->npartial, h->dscalar, h->stream);
+                                                  h->npartial, (unsigned*)(h->uscalar + 1), res, h->stream);
   if (e != cudaSuccess) throw mxm::CudaError(e, "reduction launch");
-  CK(cudaMemcpyAsync(out, h->dscalar, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
+  mxm::fetch_result(h, out);
   if (!(*out == *out) || *out > 1.0e300 || *out < -1.0e300) {
     h->err = "non-finite reduction result";
     return MXM_DG_ENONFINITE;
@@ -1284,14 +1322,17 @@ int mxm_dg_reduce_conserved_noalloc(void* handle, int which, int c, int kind, in
   const int nb = nblocks > 0 ? nblocks : int(want < h->npartial ? want : h->npartial);
   const double scale = mxm::reduce_scale(h, kind);
   double* result = scratch + mxm::kStaticPartials;
+  // (two callers that race here may leave the counter anywhere: it starts each call at zero)
+  unsigned* count = (unsigned*)(result + 1);
+  CK(cudaMemsetAsync(count, 0, sizeof(unsigned), h->stream));
   const size_t off = size_t(h->own_e0()) * h->NP * h->NC;
   cudaError_t e = h->rbytes == 8
                       ? mxm::launch_reduce<double>(h->P, h->dim, h->NC, (const double*)h->q[which] + off,
                                                    (const double*)h->w, h->own_ne(), c, kind, scale, scratch, nb,
-                                                   result, h->stream)
+                                                   count, result, h->stream)
                       : mxm::launch_reduce<float>(h->P, h->dim, h->NC, (const float*)h->q[which] + off,
                                                   (const float*)h->w, h->own_ne(), c, kind, scale, scratch, nb,
-                                                  result, h->stream);
+                                                  count, result, h->stream);
   if (e != cudaSuccess) throw mxm::CudaError(e, "reduction launch");
   CK(cudaMemcpyAsync(out, result, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));

@@ -270,13 +270,49 @@ struct LimArgs {
   R eps2;
 };
 
+// Where a reduction over the whole grid ends: every block leaves its share in
+// `acc` (maxima) or `partial`, and the block that counts last finishes the
+// result, writes it to `out` (device memory, or host memory the device can
+// write) and leaves acc and count at zero for the next reduction.  One launch,
+// and with host memory no copy: a call that returns a number to the host is
+// its launch and one synchronisation.
+struct ReduceOut {
+  unsigned long long* acc;
+  unsigned* count;
+  double* out;
+};
+#ifdef __CUDACC__
+// Whether this block is the last of the grid to get here (every thread of
+// the block calls it, after its writes); the counter is zero again after.
+__device__ __forceinline__ bool last_block(unsigned* count) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicInc(count, gridDim.x - 1) == gridDim.x - 1;
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+// Largest `best` (>= 0) over the grid: IEEE bit patterns of non-negative
+// doubles order like unsigned integers, so atomicMax on the bits gives an
+// order-independent (deterministic) maximum.
+__device__ __forceinline__ void grid_max(double best, const ReduceOut& r) {
+  for (int o = 16; o > 0; o >>= 1) best = fmax(best, __shfl_xor_sync(0xffffffffu, best, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(r.acc, (unsigned long long)__double_as_longlong(best));
+  if (last_block(r.count) && threadIdx.x == 0) {
+    *r.out = __longlong_as_double((long long)atomicExch(r.acc, 0ull));
+    __threadfence_system();
+  }
+}
+#endif
+
 // Host launchers; each is explicitly instantiated next to its kernels.
 template <class R, class Phys>
 cudaError_t launch_stage3d(int P, const Stage3DArgs<R>& a, const KuhnTab3<R>& tab, const Phys& ph, int nsm,
                            cudaStream_t st);
 template <class R, class Phys>
 cudaError_t launch_wavespeed3d(int P, const Stage3DArgs<R>& a, const KuhnTab3<R>& tab, const Phys& ph,
-                               unsigned long long* out, cudaStream_t st);
+                               const ReduceOut& out, cudaStream_t st);
 // Batched tensor-core 3D stage: the tiles of many solves of one physics,
 // order and operand kind in one launch.  items[t] = {solve, first cell,
 // cells, 0}, the tiles of one solve consecutive; margs[solve] are the
@@ -308,13 +344,13 @@ template <class R, class Phys>
 cudaError_t launch_stage2d(int P, const Stage2DArgs<R>& a, const KuhnTab2<R>& tab, const Phys& ph, int nsm,
                            cudaStream_t st);
 template <class R, class Phys>
-cudaError_t launch_wavespeed2d(const R* q, int64_t nnodes, const Phys& ph, unsigned long long* out, cudaStream_t st);
+cudaError_t launch_wavespeed2d(const R* q, int64_t nnodes, const Phys& ph, const ReduceOut& out, cudaStream_t st);
 template <class R>
 cudaError_t launch_limiter(int dim, int P, int NC, const LimArgs<R>& a, const KuhnTab3<R>& t3, const KuhnTab2<R>& t2,
                            cudaStream_t st);
 template <class R>
 cudaError_t launch_reduce(int P, int dim, int NC, const R* q, const R* w, int64_t ne, int c, int kind, double scale,
-                          double* partial, int npartial, double* out, cudaStream_t st);
+                          double* partial, int npartial, unsigned* count, double* out, cudaStream_t st);
 // Static (module-resident) scratch of the allocation-free reduction: the
 // address of kStaticPartials partial slots followed by the result slot, on
 // the calling thread's current device.

@@ -67,7 +67,8 @@ struct Handle {
   float* xyz = nullptr;
   double* partial = nullptr;
   double* dscalar = nullptr;
-  unsigned long long* uscalar = nullptr;
+  unsigned long long* uscalar = nullptr;  // [0] grid maximum, [1] block counter; zero between calls
+  double* hres = nullptr;  // result word in host memory (host_slot_take), or null
   int* derr = nullptr;  // device error word written by bounded waits
   bool use_tc = false;  // MIXED / MIXED_TF32 precision: tensor-core contraction
   int tc_kind = 0;      // TC_BF16 or TC_TF32 operands
@@ -136,6 +137,9 @@ int tc_tile_cubes(int P, int NC, int kind);
 // `which` on the handle's stream; release the link
 void nccl_exchange(Handle* h, int which, cudaStream_t st);
 void nccl_release(Handle* h);
+double* host_slot_take();
+void host_slot_give(double* p);
+void fetch_result(Handle* h, double* out);
 void fill_ic(Handle* h, int which, int kind, const double* params, int nparams);
 // 2D GLM-MHD psi damping after each step: whether h has it, and its factor
 bool glm_damped(const Handle* h);

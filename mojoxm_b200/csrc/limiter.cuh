@@ -273,9 +273,11 @@ __global__ void __launch_bounds__(kLimBlock) theta3d_batch_kernel(LimBatch3<R> l
   }
 }
 
-// ---- FP64 reductions: per-block partial sums, then a fixed-order final sum.
+// ---- FP64 reductions: per-block partial sums, then the last block's sum of
+// them in a fixed order.
 template <class R, int NP, int NC>
-__global__ void reduce_partial_kernel(const R* q, const R* w, int64_t ne, int c, int kind, double* partial) {
+__global__ void reduce_kernel(const R* q, const R* w, int64_t ne, int c, int kind, double scale, double* partial,
+                              unsigned* count, double* out) {
   __shared__ double red[32];
   double acc = kind == 2 ? 0.0 : 0.0;
   for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < ne; e += int64_t(gridDim.x) * blockDim.x) {
@@ -304,8 +306,21 @@ __global__ void reduce_partial_kernel(const R* q, const R* w, int64_t ne, int c,
     for (int k = 0; k < int(blockDim.x >> 5); ++k) s = kind == 2 ? fmax(s, red[k]) : s + red[k];
     partial[blockIdx.x] = s;
   }
+  if (!last_block(count) || threadIdx.x >= 32) return;
+  // one warp, fixed order: deterministic
+  double s = 0.0;
+  for (int k = threadIdx.x; k < int(gridDim.x); k += 32) {
+    const double v = __ldcg(&partial[k]);
+    s = kind == 2 ? fmax(s, v) : s + v;
+  }
+  red[threadIdx.x] = s;
+  __syncwarp();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int k = 0; k < 32; ++k) t = kind == 2 ? fmax(t, red[k]) : t + red[k];
+    *out = t * scale;
+    __threadfence_system();
+  }
 }
-
-__global__ void reduce_final_kernel(const double* partial, int n, int kind, double scale, double* out);
 
 }  // namespace mxm

@@ -358,19 +358,18 @@ cudaError_t launch_stage2d(int P, const Stage2DArgs<R>& a, const KuhnTab2<R>& ta
 
 // Nodal max of the physical signal speed (2D kernels return no face speed).
 template <class R, class Phys, int NC>
-__global__ void wavespeed2d_kernel(const R* q, int64_t nnodes, Phys ph, unsigned long long* out) {
+__global__ void wavespeed2d_kernel(const R* q, int64_t nnodes, Phys ph, ReduceOut out) {
   const int64_t n = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   double best = 0.0;
   if (n < nnodes) {
     best = double(ph.speed(q + n * NC));
     if (!(best >= 0.0)) best = __longlong_as_double(0x7ff0000000000000LL);
   }
-  for (int o = 16; o > 0; o >>= 1) best = fmax(best, __shfl_xor_sync(0xffffffffu, best, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(best));
+  grid_max(best, out);
 }
 
 template <class R, class Phys>
-cudaError_t launch_wavespeed2d(const R* q, int64_t nnodes, const Phys& ph, unsigned long long* out, cudaStream_t st) {
+cudaError_t launch_wavespeed2d(const R* q, int64_t nnodes, const Phys& ph, const ReduceOut& out, cudaStream_t st) {
   wavespeed2d_kernel<R, Phys, Phys::NC><<<int((nnodes + 255) / 256), 256, 0, st>>>(q, nnodes, ph, out);
   return cudaGetLastError();
 }
@@ -378,6 +377,6 @@ cudaError_t launch_wavespeed2d(const R* q, int64_t nnodes, const Phys& ph, unsig
 #define MXM_INSTANTIATE_STAGE2D(R, PHYS)                                                                          \
   template cudaError_t launch_stage2d<R, PHYS>(int, const Stage2DArgs<R>&, const KuhnTab2<R>&, const PHYS&, int, \
                                                cudaStream_t);                                                     \
-  template cudaError_t launch_wavespeed2d<R, PHYS>(const R*, int64_t, const PHYS&, unsigned long long*, cudaStream_t);
+  template cudaError_t launch_wavespeed2d<R, PHYS>(const R*, int64_t, const PHYS&, const ReduceOut&, cudaStream_t);
 
 }  // namespace mxm

@@ -342,11 +342,9 @@ __global__ void __launch_bounds__(NT) stage3d_kernel(Stage3DArgs<R> args, KuhnTa
 
 // Max over every element face node of the signal speed that
 // numerical_flux / boundary_flux return (the reference discards it at
-// src/solver.mojo:266-268); one thread per (element, face node).  Speeds are
-// non-negative, so their IEEE bit patterns order like unsigned integers and
-// atomicMax on the bits gives an order-independent (deterministic) max.
+// src/solver.mojo:266-268); one thread per (element, face node).
 template <class R, class Phys, int P>
-__global__ void wavespeed3d_kernel(Stage3DArgs<R> args, KuhnTab3<R> tab, Phys ph, unsigned long long* out) {
+__global__ void wavespeed3d_kernel(Stage3DArgs<R> args, KuhnTab3<R> tab, Phys ph, ReduceOut out) {
   constexpr int NC = Phys::NC, NP = ntet(P), NFP = ntri(P);
   const int64_t tid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   double best = 0.0;
@@ -377,8 +375,7 @@ __global__ void wavespeed3d_kernel(Stage3DArgs<R> args, KuhnTab3<R> tab, Phys ph
     best = double(s);
     if (!(best >= 0.0)) best = __longlong_as_double(0x7ff0000000000000LL);  // NaN -> +inf flags it
   }
-  for (int o = 16; o > 0; o >>= 1) best = fmax(best, __shfl_xor_sync(0xffffffffu, best, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(best));
+  grid_max(best, out);
 }
 
 template <class R, int P, int NC, int EC, bool ASMEM>

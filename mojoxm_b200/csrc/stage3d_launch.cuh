@@ -83,7 +83,7 @@ cudaError_t launch_stage3d(int P, const Stage3DArgs<R>& a, const KuhnTab3<R>& ta
 
 template <class R, class Phys>
 cudaError_t launch_wavespeed3d(int P, const Stage3DArgs<R>& a, const KuhnTab3<R>& tab, const Phys& ph,
-                               unsigned long long* out, cudaStream_t st) {
+                               const ReduceOut& out, cudaStream_t st) {
   const int64_t n = int64_t(a.ncell - a.cbeg) * 6 * 4 * ntri(P);
   const int nb = int((n + 255) / 256);
   switch (P) {
@@ -101,6 +101,6 @@ cudaError_t launch_wavespeed3d(int P, const Stage3DArgs<R>& a, const KuhnTab3<R>
   template cudaError_t launch_stage3d<R, PHYS>(int, const Stage3DArgs<R>&, const KuhnTab3<R>&, const PHYS&, int, \
                                                cudaStream_t);                                                     \
   template cudaError_t launch_wavespeed3d<R, PHYS>(int, const Stage3DArgs<R>&, const KuhnTab3<R>&, const PHYS&,  \
-                                                   unsigned long long*, cudaStream_t);
+                                                   const ReduceOut&, cudaStream_t);
 
 }  // namespace mxm
