@@ -317,6 +317,8 @@ Stage3DArgs<R> stage3d_args(const Handle* h, const void* qi, const void* qa, con
   for (int k = 0; k < 6; ++k) ar.bc[k] = h->bc[k];
   ar.rhs_only = rhs_only;
   ar.err = h->derr;
+  ar.tab = h->use_tc ? nullptr : (const KuhnTab3<R>*)((const unsigned char*)h->A + h->tab_off);
+  ar.ec = 0;
   ar.tctab = h->use_tc ? (const Tc3Tab*)((const unsigned char*)h->tcimg + h->tctab_off) : nullptr;
   return ar;
 }
@@ -355,14 +357,13 @@ cudaError_t stage_launch(Handle* h, const void* qi, const void* qa, const void* 
   const R cdt = R(c * dt);
   if (h->dim == 3) {
     const Stage3DArgs<R> ar = stage3d_args<R>(h, qi, qa, qb, qo, b, c, dt, rhs_only, c0, c1);
-    const KuhnTab3<R>& t = tab3<R>(h);
     // MIXED precision routes the 3D stage through the tensor-core kernel
     return with_phys3d<R>(h, [&](const auto& ph) -> cudaError_t {
       if constexpr (std::is_same<R, float>::value && std::decay<decltype(ph)>::type::NC <= 16) {
         if (h->use_tc)
           return launch_stage3d_tc(h->P, h->tc_kind, ar, ph, (const unsigned char*)h->tcimg, h->nsm, h->stream);
       }
-      return launch_stage3d<R>(h->P, ar, t, ph, h->nsm, h->stream);
+      return launch_stage3d<R>(h->P, ar, ph, h->nsm, h->stream);
     });
   }
   Stage2DArgs<R> ar;
@@ -937,18 +938,25 @@ Handle* create(const mxm_dg_mesh_desc* m, const mxm_dg_physics_desc* ph, int P, 
     std::vector<double> At(size_t(raw->K) * raw->NP);  // k-major copy of the shared operator
     for (int i = 0; i < raw->NP; ++i)
       for (int k = 0; k < raw->K; ++k) At[size_t(k) * raw->NP + i] = raw->Ahost[size_t(i) * raw->K + k];
-    auto upload = [&](void** dst, const std::vector<double>& src) {
-      dev_alloc(raw, dst, src.size() * raw->rbytes);
-      if (raw->rbytes == 8) {
-        CK(cudaMemcpyAsync(*dst, src.data(), src.size() * 8, cudaMemcpyHostToDevice, raw->stream));
-      } else {
-        std::vector<float> f(src.begin(), src.end());
-        CK(cudaMemcpyAsync(*dst, f.data(), f.size() * 4, cudaMemcpyHostToDevice, raw->stream));
-        CK(cudaStreamSynchronize(raw->stream));  // f goes out of scope
-      }
+    // each array goes up in the handle's real type, followed (16-byte
+    // aligned) by `extra` bytes as they are
+    auto upload = [&](void** dst, const std::vector<double>& src, const void* extra, size_t nextra) -> size_t {
+      const size_t off = (src.size() * raw->rbytes + 15) / 16 * 16;
+      std::vector<unsigned char> buf(off + (nextra + 15) / 16 * 16, 0);
+      if (raw->rbytes == 8) std::memcpy(buf.data(), src.data(), src.size() * 8);
+      else
+        for (size_t i = 0; i < src.size(); ++i) reinterpret_cast<float*>(buf.data())[i] = float(src[i]);
+      if (nextra) std::memcpy(&buf[off], extra, nextra);
+      dev_alloc(raw, dst, buf.size());
+      CK(cudaMemcpyAsync(*dst, buf.data(), buf.size(), cudaMemcpyHostToDevice, raw->stream));
+      CK(cudaStreamSynchronize(raw->stream));  // buf goes out of scope
+      return off;
     };
-    upload(&raw->A, At);
-    upload(&raw->w, raw->ref.w);
+    // the 3D table follows the operator
+    const void* tab = raw->rbytes == 8 ? (const void*)&raw->t3d : (const void*)&raw->t3f;
+    const size_t tab_bytes = raw->dim != 3 ? 0 : (raw->rbytes == 8 ? sizeof(raw->t3d) : sizeof(raw->t3f));
+    raw->tab_off = upload(&raw->A, At, tab, tab_bytes);
+    upload(&raw->w, raw->ref.w, nullptr, 0);
     if (raw->use_tc) {
       auto img = tc_operator_image(raw->Ahost, raw->NP, raw->K, 3 * raw->NP, raw->tc_kind);
       raw->tctab_off = (img.size() + 15) / 16 * 16;

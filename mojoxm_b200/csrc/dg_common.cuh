@@ -92,8 +92,8 @@ __host__ __device__ constexpr size_t stage3d_smem(int P, int NC, int rb, int EC,
   const size_t tab = rb == 8 ? (sizeof(KuhnTab3<double>) + 15) / 16 * 16 : (sizeof(KuhnTab3<float>) + 15) / 16 * 16;
   const size_t NP = size_t(ntet(P)), K = size_t(3 * ntet(P) + 4 * ntri(P));
   return 16 + tab + size_t(rb) * (2 * size_t(6 * EC) * NP * NC + size_t(6 * EC) * stage3d_bstr(P, NC, rb) +
-                                  (asmem ? K * NP : 0)) +
-         size_t(EC) * 12 * sizeof(int);
+                                  (asmem ? (K * NP + 1) / 2 * 2 : 0)) +
+         size_t(EC) * 6 * sizeof(int2);
 }
 // Least shared memory the 3D SIMT stage needs (one cube per tile, operator
 // read from global memory).
@@ -237,6 +237,8 @@ struct Stage3DArgs {
   int rhs_only;
   int* err;  // device error word (bounded waits that gave up set bit 0)
   const Tc3Tab* tctab;  // tensor-core stage: its topology table (null otherwise)
+  const KuhnTab3<R>* tab;  // vector stage: the table in device memory (null otherwise)
+  int ec;  // vector stage: cubes per tile, at most the kernel's EC (set by the launch)
 };
 
 template <class R>
@@ -308,8 +310,7 @@ __device__ __forceinline__ void grid_max(double best, const ReduceOut& r) {
 
 // Host launchers; each is explicitly instantiated next to its kernels.
 template <class R, class Phys>
-cudaError_t launch_stage3d(int P, const Stage3DArgs<R>& a, const KuhnTab3<R>& tab, const Phys& ph, int nsm,
-                           cudaStream_t st);
+cudaError_t launch_stage3d(int P, const Stage3DArgs<R>& a, const Phys& ph, int nsm, cudaStream_t st);
 template <class R, class Phys>
 cudaError_t launch_wavespeed3d(int P, const Stage3DArgs<R>& a, const KuhnTab3<R>& tab, const Phys& ph,
                                const ReduceOut& out, cudaStream_t st);

@@ -61,7 +61,8 @@ struct Handle {
   int device = 0, nsm = 148;
   cudaStream_t stream = nullptr;
   void* q[3] = {nullptr, nullptr, nullptr};
-  void* A = nullptr;
+  void* A = nullptr;   // operator; in 3D the topology table follows at tab_off
+  size_t tab_off = 0;
   void* w = nullptr;
   void* avg = nullptr;
   float* xyz = nullptr;

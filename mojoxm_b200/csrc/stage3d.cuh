@@ -27,7 +27,7 @@
 //  * q_a / q_b equal to q_in (SSPRK3 stages 1-3) are read from the tile, so
 //    each stage moves the algorithmic minimum of state bytes.
 //  * Where a tile's contraction works (element x RI-row group) would leave
-//    most of the block idle (one-cube tiles at P4/P5 in FP64), KS lanes of
+//    most of the block idle (FP32 P4 / P5), KS lanes of
 //    a warp share a work, each summing every KS-th K column, and a shuffle
 //    butterfly (ks_fold) gives each lane complete rows for the epilogue.
 #pragma once
@@ -83,8 +83,28 @@ __device__ __forceinline__ void ks_fold(R (&acc)[RI][NC], unsigned gmask, int la
   }
 }
 
+// FP64 contraction on the tensor cores (mma.sync f64; tcgen05 has no FP64
+// kind): D += A B of 8 operator rows x 4 columns and 4 x 8 (element,
+// component) columns.
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
+
+// Shape of the FP64 contraction of a tile: its (element, component) columns
+// in groups of 8, the operator's rows in groups of 8 (MT), MG of them a task;
+// rows are split over tasks only as far as the block's warps need works.
+template <int NP, int COLS, int NW>
+struct DmmaShape {
+  static constexpr int NTL = (COLS + 7) / 8, MT = (NP + 7) / 8;
+  static constexpr int split(int s) { return NTL * s >= NW || s >= MT ? s : split(s + 1); }
+  static constexpr int MG = (MT + split(1) - 1) / split(1), MS = (MT + MG - 1) / MG;
+  static constexpr int TASKS = NTL * MS, ROUNDS = (TASKS + NW - 1) / NW;
+};
+
 template <class R, class Phys, int P, int EC, int RI, int KS, int NT, bool ASMEM>
-__global__ void __launch_bounds__(NT) stage3d_kernel(Stage3DArgs<R> args, KuhnTab3<R> tabp, Phys ph) {
+__global__ void __launch_bounds__(NT) stage3d_kernel(Stage3DArgs<R> args, Phys ph) {
   constexpr int NC = Phys::NC;
   using S = Stage3DShape<P, NC, R>;
   constexpr int NP = S::NP, NFP = S::NFP, K = S::K, BSTR = S::BSTR;
@@ -104,29 +124,35 @@ __global__ void __launch_bounds__(NT) stage3d_kernel(Stage3DArgs<R> args, KuhnTa
   R* sQ = reinterpret_cast<R*>(smem_raw + 16 + kTabBytes);                     // [2][QV]
   R* sB = sQ + 2 * QV;                                                         // [EB][BSTR]
   R* sA = sB + EB * BSTR;                                                      // [K][NP] (ASMEM)
-  int* sNb = reinterpret_cast<int*>(sA + (ASMEM ? K * NP : 0));                // [EC][6] neighbour cubes
-  int* sMd = sNb + EC * 6;                                                     // [EC][6] face modes
+  // [EC][6] {neighbour cube, face mode | code << 8}
+  int2* sCd = reinterpret_cast<int2*>(sA + (ASMEM ? (K * NP + 1) / 2 * 2 : 0));
   const R* Aop = ASMEM ? sA : args.A;
 
   const int tid = threadIdx.x;
   grid_dep_launch();  // the next stage may set up as this one's blocks finish
-  const int ngroups = (args.ncell - args.cbeg + EC - 1) / EC;
+  const int ec = args.ec, ngroups = (args.ncell - args.cbeg + ec - 1) / ec;  // ec <= EC cubes a tile
   if (tid == 0) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
     fence_mbar_init();
   }
   {
-    const int* src = reinterpret_cast<const int*>(&tabp);
-    int* dst = reinterpret_cast<int*>(tab);
-    for (int k = tid; k < int(sizeof(KuhnTab3<R>) / 4); k += NT) dst[k] = src[k];
+    const uint4* src = reinterpret_cast<const uint4*>(args.tab);
+    uint4* dst = reinterpret_cast<uint4*>(tab);
+    for (int k = tid; k < int(kTabBytes / 16); k += NT) dst[k] = src[k];
   }
-  if (ASMEM)
+  if constexpr (ASMEM && kAOff % 16 == 0) {
+    const uint4* src = reinterpret_cast<const uint4*>(args.A);
+    constexpr int N = NP * K * int(sizeof(R)) / 16;
+    for (int k = tid; k < N; k += NT) reinterpret_cast<uint4*>(sA)[k] = src[k];
+    for (int k = N * 16 / int(sizeof(R)) + tid; k < NP * K; k += NT) sA[k] = args.A[k];
+  } else if (ASMEM) {
     for (int idx = tid; idx < NP * K; idx += NT) sA[idx] = args.A[idx];
+  }
   __syncthreads();
 
   auto issue = [&](int grp, int buf) {
-    const int c0 = args.cbeg + grp * EC, nc = min(EC, args.ncell - c0);
+    const int c0 = args.cbeg + grp * ec, nc = min(ec, args.ncell - c0);
     const uint32_t bytes = uint32_t(nc) * 6u * NP * NC * sizeof(R);
     fence_proxy_async();
     mbar_arrive_expect_tx(&bar[buf], bytes);
@@ -139,9 +165,9 @@ __global__ void __launch_bounds__(NT) stage3d_kernel(Stage3DArgs<R> args, KuhnTa
   // (whole tiles of the usual shapes; a partial last tile may take plain loads)
   auto tile_bulk = [&](int g) -> bool {
     const size_t per_cube = size_t(6) * NP * NC * sizeof(R);
-    const int cg = args.cbeg + g * EC;
+    const int cg = args.cbeg + g * ec;
     const size_t start = reinterpret_cast<uintptr_t>(args.q_in) + size_t(cg) * per_cube;
-    const size_t bytes = size_t(min(EC, args.ncell - cg)) * per_cube;
+    const size_t bytes = size_t(min(ec, args.ncell - cg)) * per_cube;
     return start % 16 == 0 && bytes % 16 == 0;
   };
   uint32_t par = 0u;  // bit b: phase parity of tile buffer b
@@ -152,10 +178,9 @@ __global__ void __launch_bounds__(NT) stage3d_kernel(Stage3DArgs<R> args, KuhnTa
   grid_dep_wait();
   if (tid == 0 && int(blockIdx.x) < ngroups && tile_bulk(blockIdx.x)) issue(blockIdx.x, 0);
 
-  const int nwork = tab->n_face_work;
   for (int grp = blockIdx.x; grp < ngroups; grp += gridDim.x, buf ^= 1) {
-    const int cell0 = args.cbeg + grp * EC;
-    const int nhere = min(EC, args.ncell - cell0);
+    const int cell0 = args.cbeg + grp * ec;
+    const int nhere = min(ec, args.ncell - cell0);
     const int ne_here = 6 * nhere;
     R* q = sQ + buf * QV;
     if (tile_bulk(grp)) {
@@ -176,9 +201,7 @@ __global__ void __launch_bounds__(NT) stage3d_kernel(Stage3DArgs<R> args, KuhnTa
     }
     for (int w = tid; w < nhere * 6; w += NT) {
       const int cl = w / 6, dd = w - cl * 6;
-      const int2 cd = cube_dir3(cell0 + cl, args.nx, args.ny, args.nz, args.bc, dd);
-      sNb[w] = cd.x;
-      sMd[w] = cd.y;
+      sCd[w] = cube_dir3(cell0 + cl, args.nx, args.ny, args.nz, args.bc, dd);
     }
     __syncthreads();
     // ---- volume fluxes in reference coordinates -> B rows k*NP + j
@@ -195,18 +218,17 @@ __global__ void __launch_bounds__(NT) stage3d_kernel(Stage3DArgs<R> args, KuhnTa
           b[k * NP * NC + c] = iJ[k * 3 + 0] * F[c] + iJ[k * 3 + 1] * F[NC + c] + iJ[k * 3 + 2] * F[2 * NC + c];
     }
     // ---- face numerical fluxes, scaled by side*area/(6V) -> B rows 3NP + lf*NFP + m
-    for (int idx = tid; idx < EC * nwork * NFP; idx += NT) {
-      const int cl = idx % EC, rest = idx / EC, m = rest % NFP, wk = rest / NFP;
-      if (cl >= nhere) continue;
+    for (int idx = tid; idx < nhere * kFaceWork3 * NFP; idx += NT) {
+      const int rest = idx / NFP, m = idx - rest * NFP, cl = rest / kFaceWork3, wk = rest - cl * kFaceWork3;
       const int tl = tab->face_work[wk], t = tl >> 2, lf = tl & 3;
       const int el = cl * 6 + t, ax = tab->axis[t][lf], nbt = tab->nb_t[t][lf];
       int mode = FACE_INTERIOR, code = 0, nbcube = 0;
       if (ax >= 0) {
         const int dd = 2 * ax + (tab->dir[t][lf] > 0 ? 1 : 0);
-        const int md = sMd[cl * 6 + dd];
-        mode = md & 0xff;
-        code = md >> 8;
-        nbcube = sNb[cl * 6 + dd];
+        const int2 cd = sCd[cl * 6 + dd];
+        mode = cd.y & 0xff;
+        code = cd.y >> 8;
+        nbcube = cd.x;
       }
       const R* qo = &q[(el * NP + tab->own_node[lf][m]) * NC];
       R nx = tab->normal[t][lf][0], ny = tab->normal[t][lf][1], nz = tab->normal[t][lf][2];
@@ -261,10 +283,88 @@ __global__ void __launch_bounds__(NT) stage3d_kernel(Stage3DArgs<R> args, KuhnTa
       }
     }
     __syncthreads();
-    // ---- contraction rhs = A B, source, RK combine, floor, store.  A work
-    // is an RI x NC tile of one element; KS consecutive lanes share it, each
-    // summing every KS-th K column, and ks_fold hands each lane its rows.
-    const bool a_in = args.q_a == args.q_in, b_in = args.q_b == args.q_in;
+    // ---- contraction rhs = A B, source, RK combine (every stage's q_b is
+    // its q_in), floor, store
+    const bool a_in = args.q_a == args.q_in;
+    if constexpr (sizeof(R) == 8) {
+      // FP64: a warp multiplies MG groups of 8 operator rows with 8 (element,
+      // component) columns, four K columns at a time.  The vector form
+      // (2 rows x NC a thread) read 7 shared values per 10 products and took
+      // 230 of 504 us a stage at 32^3 P3 Euler; a stage takes 405 us now
+      // (24^3 P4 647 -> 415, 16^3 P5 551 -> 420, 32^3 P2 232 -> 210).
+      using D = DmmaShape<NP, 6 * EC * NC, NT / 32>;
+      const int warp = tid >> 5, lane = tid & 31, ncols = ne_here * NC;
+      double acc[D::ROUNDS][D::MG][2];
+#pragma unroll
+      for (int r = 0; r < D::ROUNDS; ++r) {
+#pragma unroll
+        for (int g = 0; g < D::MG; ++g) acc[r][g][0] = acc[r][g][1] = 0.0;
+        const int task = warp + r * (NT / 32), col0 = task % D::NTL * 8, mt0 = task / D::NTL * D::MG;
+        if (task >= D::TASKS || col0 >= ncols) continue;  // (warp-uniform)
+        // this lane's column and rows (clamped: rows past NP and columns past
+        // the tile go nowhere)
+        const int col = min(col0 + (lane >> 2), ncols - 1), el = col / NC;
+        const R* b = sB + el * BSTR + (col - el * NC);
+        const R* arow[D::MG];
+#pragma unroll
+        for (int g = 0; g < D::MG; ++g) arow[g] = Aop + min((mt0 + g) * 8 + (lane >> 2), NP - 1);
+#pragma unroll 4
+        for (int k = lane & 3; k < K / 4 * 4; k += 4) {
+          const double bv = b[k * NC];
+#pragma unroll
+          for (int g = 0; g < D::MG; ++g) dmma(acc[r][g], ASMEM ? arow[g][k * NP] : __ldg(&arow[g][k * NP]), bv);
+        }
+        if constexpr (K % 4 != 0) {
+          const int k = K / 4 * 4 + (lane & 3);
+          const bool in = k < K;
+          const double bv = in ? b[k * NC] : 0.0;
+#pragma unroll
+          for (int g = 0; g < D::MG; ++g)
+            dmma(acc[r][g], in ? (ASMEM ? arow[g][k * NP] : __ldg(&arow[g][k * NP])) : 0.0, bv);
+        }
+      }
+      __syncthreads();  // the operands have been read: rhs takes their place, node by node
+#pragma unroll
+      for (int r = 0; r < D::ROUNDS; ++r) {
+        const int task = warp + r * (NT / 32), col0 = task % D::NTL * 8, mt0 = task / D::NTL * D::MG;
+        if (task >= D::TASKS) continue;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int col = col0 + 2 * (lane & 3) + h, el = col / NC;
+          if (col >= ncols) continue;
+#pragma unroll
+          for (int g = 0; g < D::MG; ++g) {
+            const int i = (mt0 + g) * 8 + (lane >> 2);
+            if (i < NP) sB[el * BSTR + i * NC + (col - el * NC)] = acc[r][g][h];
+          }
+        }
+      }
+      __syncthreads();
+      for (int idx = tid; idx < ne_here * NP; idx += NT) {
+        const int el = idx / NP, i = idx - el * NP;
+        const size_t base = (size_t(cell0) * 6 * NP + idx) * NC;
+        const R* ql = &q[idx * NC];
+        const R* rh = &sB[el * BSTR + i * NC];
+        R src[NC], out[NC];
+        if (Phys::kSource) ph.source(ql, src);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          const R rhs = Phys::kSource ? rh[c] + src[c] : rh[c];
+          if (args.rhs_only) {
+            out[c] = rhs;
+          } else {
+            const R vb = ql[c], va = a_in ? vb : args.q_a[base + c];
+            out[c] = va + args.b * (vb - va) + args.cdt * rhs;
+          }
+        }
+        if (Phys::kLimit && !args.rhs_only) ph.limit(out);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) args.q_out[base + c] = out[c];
+      }
+    } else {
+    // FP32: a work is an RI x NC tile of one element; KS consecutive lanes
+    // share it, each summing every KS-th K column, and ks_fold hands each
+    // lane its rows.
     constexpr int RO = ks_rows(RI, KS / 2);
     for (int w = tid; w < ne_here * G * KS; w += NT) {
       const int wk = w / KS, s = w - wk * KS;
@@ -327,8 +427,7 @@ __global__ void __launch_bounds__(NT) stage3d_kernel(Stage3DArgs<R> args, KuhnTa
           if (args.rhs_only) {
             out[c] = rhs;
           } else {
-            const R va = a_in ? ql[c] : args.q_a[base + c];
-            const R vb = b_in ? ql[c] : args.q_b[base + c];
+            const R vb = ql[c], va = a_in ? vb : args.q_a[base + c];
             out[c] = va + args.b * (vb - va) + args.cdt * rhs;
           }
         }
@@ -336,6 +435,7 @@ __global__ void __launch_bounds__(NT) stage3d_kernel(Stage3DArgs<R> args, KuhnTa
 #pragma unroll
         for (int c = 0; c < NC; ++c) args.q_out[base + c] = out[c];
       }
+    }
     }
   }
 }

@@ -25,10 +25,10 @@ template <class R, int P, int NC>
 struct Cfg3 {
   using S = Stage3DShape<P, NC, R>;
   static constexpr int NP = S::NP;
-  // rows per thread: a divisor of NP (fewer for wide states)
-  static constexpr int RI0 = sizeof(R) == 8 ? (P <= 3 ? 2 : (P == 4 ? 5 : 4))
-                                            : (P == 1 ? 4 : (P == 2 ? 5 : (P == 3 ? 4 : (P == 4 ? 5 : 8))));
-  static constexpr int RI = NC > 6 ? ri_capped(RI0, NP, NC, sizeof(R) == 8 ? 48 : 64) : RI0;
+  // FP32: rows per thread of the contraction, a divisor of NP (fewer for wide
+  // states); FP64 contracts on the tensor cores
+  static constexpr int RI0 = P == 1 ? 4 : (P == 2 ? 5 : (P == 3 ? 4 : (P == 4 ? 5 : 8)));
+  static constexpr int RI = sizeof(R) == 8 ? 1 : (NC > 6 ? ri_capped(RI0, NP, NC, 64) : RI0);
   // keep the shared operator in shared memory when it takes <= 64 KB and a
   // one-cube tile still fits beside it
   static constexpr bool ASMEM = sizeof(R) * S::K * S::NP <= 64 * 1024 &&
@@ -39,17 +39,16 @@ struct Cfg3 {
   static constexpr int EC_RAW = kBudget > kFixed ? int((kBudget - kFixed) / kPerCube) : 1;
   static constexpr int EC = EC_RAW > 16 ? 16 : (EC_RAW < 1 ? 1 : EC_RAW);
   static constexpr int NT = 256;
-  // split K only where a tile's works leave most of the block idle: with
-  // 120 of 256 threads busy (FP64 P3) a 2-way split measured -4 %, with 126
-  // (FP32 P4) +9 %, with 42 (FP64 P4) +69 %
+  // FP32: split K where a tile's works leave at least half of the block idle
+  // (126 of 256 threads busy, P4: +9 %)
   static constexpr int WORKS = 6 * EC * (S::NP / RI);
-  static constexpr int KS = (sizeof(R) == 8 ? WORKS * 8 < 3 * NT : WORKS * 2 <= NT) ? ks_pick(WORKS, NT, S::K) : 1;
+  static constexpr int KS = sizeof(R) == 4 && WORKS * 2 <= NT ? ks_pick(WORKS, NT, S::K) : 1;
   static constexpr size_t kSmem = stage3d_smem_bytes<R, P, NC, EC, ASMEM>();
   static constexpr bool FITS = kSmem <= kMaxSmemPerBlock;
 };
 
 template <class R, class Phys, int P>
-cudaError_t launch3_p(const Stage3DArgs<R>& a, const KuhnTab3<R>& tab, const Phys& ph, int nsm, cudaStream_t st) {
+cudaError_t launch3_p(const Stage3DArgs<R>& a, const Phys& ph, int nsm, cudaStream_t st) {
   using C = Cfg3<R, P, Phys::NC>;
   if constexpr (!C::FITS) {
     return cudaErrorInvalidConfiguration;  // refused at mxm_dg_create already
@@ -60,23 +59,29 @@ cudaError_t launch3_p(const Stage3DArgs<R>& a, const KuhnTab3<R>& tab, const Phy
     cudaError_t e = persistent_blocks_per_sm((const void*)kern, C::NT, C::kSmem, &bps);
     if (e != cudaSuccess) return e;
   }
-  const int ngroups = (a.ncell - a.cbeg + C::EC - 1) / C::EC;
-  int nblk = nsm * bps;
+  // Cubes per tile: as many as fit, fewer where the mesh would leave resident
+  // blocks without a tile (the phases of a tile are short chains, so a small
+  // mesh is done sooner on more SMs: Euler FP64 P2 8^3 16.2 -> 11.7 us a
+  // stage, P3 12^3 31.8 -> 25.2, FP32 P3 10^3 19.2 -> 14.2)
+  const int ncell = a.ncell - a.cbeg, slots = nsm * bps, spread = (ncell + slots - 1) / slots;
+  Stage3DArgs<R> args = a;
+  args.ec = spread < C::EC ? (spread < 1 ? 1 : spread) : C::EC;
+  const int ngroups = (ncell + args.ec - 1) / args.ec;
+  int nblk = slots;
   if (nblk > ngroups) nblk = ngroups;
   if (nblk < 1) nblk = 1;
-  return launch_dependent(kern, nblk, C::NT, C::kSmem, st, a, tab, ph);
+  return launch_dependent(kern, nblk, C::NT, C::kSmem, st, args, ph);
   }
 }
 
 template <class R, class Phys>
-cudaError_t launch_stage3d(int P, const Stage3DArgs<R>& a, const KuhnTab3<R>& tab, const Phys& ph, int nsm,
-                           cudaStream_t st) {
+cudaError_t launch_stage3d(int P, const Stage3DArgs<R>& a, const Phys& ph, int nsm, cudaStream_t st) {
   switch (P) {
-    case 1: return launch3_p<R, Phys, 1>(a, tab, ph, nsm, st);
-    case 2: return launch3_p<R, Phys, 2>(a, tab, ph, nsm, st);
-    case 3: return launch3_p<R, Phys, 3>(a, tab, ph, nsm, st);
-    case 4: return launch3_p<R, Phys, 4>(a, tab, ph, nsm, st);
-    case 5: return launch3_p<R, Phys, 5>(a, tab, ph, nsm, st);
+    case 1: return launch3_p<R, Phys, 1>(a, ph, nsm, st);
+    case 2: return launch3_p<R, Phys, 2>(a, ph, nsm, st);
+    case 3: return launch3_p<R, Phys, 3>(a, ph, nsm, st);
+    case 4: return launch3_p<R, Phys, 4>(a, ph, nsm, st);
+    case 5: return launch3_p<R, Phys, 5>(a, ph, nsm, st);
   }
   return cudaErrorInvalidValue;
 }
@@ -98,8 +103,7 @@ cudaError_t launch_wavespeed3d(int P, const Stage3DArgs<R>& a, const KuhnTab3<R>
 }
 
 #define MXM_INSTANTIATE_STAGE3D(R, PHYS)                                                                          \
-  template cudaError_t launch_stage3d<R, PHYS>(int, const Stage3DArgs<R>&, const KuhnTab3<R>&, const PHYS&, int, \
-                                               cudaStream_t);                                                     \
+  template cudaError_t launch_stage3d<R, PHYS>(int, const Stage3DArgs<R>&, const PHYS&, int, cudaStream_t);        \
   template cudaError_t launch_wavespeed3d<R, PHYS>(int, const Stage3DArgs<R>&, const KuhnTab3<R>&, const PHYS&,  \
                                                    const ReduceOut&, cudaStream_t);
 
