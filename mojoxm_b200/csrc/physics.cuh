@@ -260,6 +260,58 @@ struct EulerD {
       flux[4] = h * ((q_l[4] + pl) * ul + (q_r[4] + pr) * ur + cmax * (q_l[4] - q_r[4]));
       return cmax;
     }
+    if constexpr (FLUX == FLUX_HLLE || FLUX == FLUX_HLLEC) {
+      if (!entropy_fix) {
+        // euler.mojo:364-485 in the world frame (the face-frame rotation pair
+        // drops out), the dissipation sum_k |s_k| W_k in terms of the jump
+        // r - l: its factors are differences already, so nothing of the
+        // states' size cancels and the waves are never formed.
+        const R rl = rho_f(q_l), rr = rho_f(q_r), il = pos_rcp(rl), ir = pos_rcp(rr);
+        const R pl = p_fi(q_l, q_l[1] * il, q_l[2] * il, q_l[3] * il);
+        const R pr = p_fi(q_r, q_r[1] * ir, q_r[2] * ir, q_r[3] * ir);
+        const R mnl = nx * q_l[1] + ny * q_l[2] + nz * q_l[3], mnr = nx * q_r[1] + ny * q_r[2] + nz * q_r[3];
+        const R ul = mnl * il, ur = mnr * ir, nn[3] = {nx, ny, nz};
+        R s0, s2;
+        {
+          const R wl = pos_sqrt(il), wr = pos_sqrt(ir), is = pos_rcp(rl * wl + rr * wr), al = wl * is, ar = wr * is;
+          const R vx = q_l[1] * al + q_r[1] * ar, vy = q_l[2] * al + q_r[2] * ar, vz = q_l[3] * al + q_r[3] * ar;
+          const R H = (q_l[4] + pl) * al + (q_r[4] + pr) * ar;
+          const R c = sqrt(rmax((gamma - R(1)) * (H - R(0.5) * (vx * vx + vy * vy + vz * vz)), R(0)));
+          const R u = vx * nx + vy * ny + vz * nz;
+          s0 = rmin(ul - pos_sqrt(gamma * pl * il), u - c);
+          s2 = rmax(ur + pos_sqrt(gamma * pr * ir), u + c);
+        }
+        const R a0 = rabs(s0), a2 = rabs(s2), h = R(0.5), el_ = q_l[4] + pl, er_ = q_r[4] + pr;
+        if constexpr (FLUX == FLUX_HLLE) {
+          const R id = pos_rcp(s2 - s0), al = (a2 - a0) * id, be = (a0 * s2 - a2 * s0) * id;
+          flux[0] = h * (mnl + mnr - (al * (mnr - mnl) + be * (q_r[0] - q_l[0])));
+#pragma unroll
+          for (int k = 1; k < 4; ++k) {
+            const R fl = q_l[k] * ul + pl * nn[k - 1], fr = q_r[k] * ur + pr * nn[k - 1];
+            flux[k] = h * (fl + fr - (al * (fr - fl) + be * (q_r[k] - q_l[k])));
+          }
+          flux[4] = h * (el_ * ul + er_ * ur - (al * (er_ * ur - el_ * ul) + be * (q_r[4] - q_l[4])));
+          return rmax(a0, a2);
+        } else {
+          // star state less its own side: q e + rho (1 + e) (s1 - un) (0, n, s1 + p / (rho (s - un))),
+          // e = (s1 - un) / (s - s1)
+          const R ml = rl * (s0 - ul), mr = rr * (s2 - ur);
+          const R s1 = (pr - pl + ul * ml - ur * mr) / (ml - mr), a1 = rabs(s1), tl = s1 - ul, tr = s1 - ur;
+          const R el = tl / (s0 - s1), er = tr / (s2 - s1), kl = (rl + rl * el) * tl, kr = (rr + rr * er) * tr;
+          const R w0 = a0 - a1, w2 = a1 - a2;
+          flux[0] = h * (mnl + mnr - (w0 * (rl * el + (rl - q_l[0])) + w2 * (rr * er + (rr - q_r[0])) +
+                                      a1 * (q_r[0] - q_l[0])));
+#pragma unroll
+          for (int k = 1; k < 4; ++k)
+            flux[k] = h * (q_l[k] * ul + q_r[k] * ur + (pl + pr) * nn[k - 1] -
+                           (w0 * (q_l[k] * el + kl * nn[k - 1]) + w2 * (q_r[k] * er + kr * nn[k - 1]) +
+                            a1 * (q_r[k] - q_l[k])));
+          flux[4] = h * (el_ * ul + er_ * ur - (w0 * (q_l[4] * el + kl * (s1 + pl / ml)) +
+                                                w2 * (q_r[4] * er + kr * (s1 + pr / mr)) + a1 * (q_r[4] - q_l[4])));
+          return rmax(rmax(a0, a1), a2);
+        }
+      }
+    }
     // tangent/binormal (euler.mojo:94-118)
     R ax = nx, ay = ny, az = nz;
     if (rabs(nx) >= R(0.9)) ay += R(1); else ax += R(1);

@@ -103,8 +103,8 @@ struct DmmaShape {
   static constexpr int TASKS = NTL * MS, ROUNDS = (TASKS + NW - 1) / NW;
 };
 
-template <class R, class Phys, int P, int EC, int RI, int KS, int NT, bool ASMEM>
-__global__ void __launch_bounds__(NT) stage3d_kernel(Stage3DArgs<R> args, Phys ph) {
+template <class R, class Phys, int P, int EC, int RI, int KS, int NT, int MINB, bool ASMEM>
+__global__ void __launch_bounds__(NT, MINB) stage3d_kernel(Stage3DArgs<R> args, Phys ph) {
   constexpr int NC = Phys::NC;
   using S = Stage3DShape<P, NC, R>;
   constexpr int NP = S::NP, NFP = S::NFP, K = S::K, BSTR = S::BSTR;

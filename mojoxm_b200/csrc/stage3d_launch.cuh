@@ -45,6 +45,11 @@ struct Cfg3 {
   static constexpr int KS = sizeof(R) == 4 && WORKS * 2 <= NT ? ks_pick(WORKS, NT, S::K) : 1;
   static constexpr size_t kSmem = stage3d_smem_bytes<R, P, NC, EC, ASMEM>();
   static constexpr bool FITS = kSmem <= kMaxSmemPerBlock;
+  // blocks per SM the register allocation allows for: two where shared memory
+  // holds two (FP64 at 24^3: HLLEC P3 361 us at 156 registers and one block, 288
+  // at 128 and two; Roe P3 392 -> 304, HLLE P2 163 -> 128); the 17-component
+  // flux would spill too much
+  static constexpr int MINB = 2 * (kSmem + 1024) <= size_t(228 * 1024) && NC <= 9 ? 2 : 1;
 };
 
 template <class R, class Phys, int P>
@@ -53,7 +58,7 @@ cudaError_t launch3_p(const Stage3DArgs<R>& a, const Phys& ph, int nsm, cudaStre
   if constexpr (!C::FITS) {
     return cudaErrorInvalidConfiguration;  // refused at mxm_dg_create already
   } else {
-  auto kern = stage3d_kernel<R, Phys, P, C::EC, C::RI, C::KS, C::NT, C::ASMEM>;
+  auto kern = stage3d_kernel<R, Phys, P, C::EC, C::RI, C::KS, C::NT, C::MINB, C::ASMEM>;
   static int bps = -1;
   if (bps < 0) {
     cudaError_t e = persistent_blocks_per_sm((const void*)kern, C::NT, C::kSmem, &bps);
