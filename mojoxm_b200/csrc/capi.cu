@@ -299,12 +299,11 @@ cudaError_t with_phys3d(const Handle* h, F&& f) {
 }
 
 template <class R>
-Stage3DArgs<R> stage3d_args(const Handle* h, const void* qi, const void* qa, const void* qb, void* qo, double b,
+Stage3DArgs<R> stage3d_args(const Handle* h, const void* qi, const void* qa, void* qo, double b,
                             double c, double dt, int rhs_only, int64_t c0, int64_t c1) {
   Stage3DArgs<R> ar;
   ar.q_in = (const R*)qi;
   ar.q_a = (const R*)qa;
-  ar.q_b = (const R*)qb;
   ar.q_out = (R*)qo;
   ar.A = (const R*)h->A;
   ar.b = R(b);
@@ -327,9 +326,9 @@ Stage3DArgs<R> stage3d_args(const Handle* h, const void* qi, const void* qa, con
 // handle as the batched 3D launch takes it.
 Stage3DArgs<float> tc_stage_args(const Handle* h, int s, double dt, int* err) {
   void *q0 = h->q[0], *q1 = h->q[1], *q2 = h->q[2];
-  Stage3DArgs<float> a = s == 0 ? stage3d_args<float>(h, q0, q0, q0, q1, 0.0, 1.0, dt, 0, h->cbeg, h->cend)
-                       : s == 1 ? stage3d_args<float>(h, q1, q0, q1, q2, 0.25, 0.25, dt, 0, h->cbeg, h->cend)
-                                : stage3d_args<float>(h, q2, q0, q2, q0, 2.0 / 3.0, 2.0 / 3.0, dt, 0, h->cbeg, h->cend);
+  Stage3DArgs<float> a = s == 0 ? stage3d_args<float>(h, q0, q0, q1, 0.0, 1.0, dt, 0, h->cbeg, h->cend)
+                       : s == 1 ? stage3d_args<float>(h, q1, q0, q2, 0.25, 0.25, dt, 0, h->cbeg, h->cend)
+                                : stage3d_args<float>(h, q2, q0, q0, 2.0 / 3.0, 2.0 / 3.0, dt, 0, h->cbeg, h->cend);
   a.err = err;
   return a;
 }
@@ -356,7 +355,7 @@ cudaError_t stage_launch(Handle* h, const void* qi, const void* qa, const void* 
   const double* p = h->phys.p;
   const R cdt = R(c * dt);
   if (h->dim == 3) {
-    const Stage3DArgs<R> ar = stage3d_args<R>(h, qi, qa, qb, qo, b, c, dt, rhs_only, c0, c1);
+    const Stage3DArgs<R> ar = stage3d_args<R>(h, qi, qa, qo, b, c, dt, rhs_only, c0, c1);
     // MIXED precision routes the 3D stage through the tensor-core kernel
     return with_phys3d<R>(h, [&](const auto& ph) -> cudaError_t {
       if constexpr (std::is_same<R, float>::value && std::decay<decltype(ph)>::type::NC <= 16) {

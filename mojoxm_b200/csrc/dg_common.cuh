@@ -221,13 +221,13 @@ template <class R>
 struct Stage3DArgs {
   const R* q_in;
   const R* q_a;
-  const R* q_b;
   R* q_out;
   const R* A;  // [K][NP] shared operator [D_r|D_s|D_t|-Lift_0..3], k-major
-  // q_out = q_a + b (q_b - q_a) + cdt rhs: the weights of q_a and q_b sum to
-  // one exactly in any precision (in FP32, a = 1/3 and b = 2/3 rounded
-  // separately sum to 1 + 3e-8, which scales the state by that much every
-  // step); cdt = c dt is rounded once from FP64.
+  // q_out = q_a + b (q_in - q_a) + cdt rhs (every Shu-Osher stage combines
+  // with its own input): the weights of q_a and q_in sum to one exactly in any
+  // precision (in FP32, a = 1/3 and b = 2/3 rounded separately sum to
+  // 1 + 3e-8, which scales the state by that much every step); cdt = c dt is
+  // rounded once from FP64.
   R b, cdt;
   int nx, ny, nz;
   // cells cbeg .. ncell-1 are computed (all cells, or the owned layers of a
@@ -317,7 +317,7 @@ cudaError_t launch_wavespeed3d(int P, const Stage3DArgs<R>& a, const KuhnTab3<R>
 // Batched tensor-core 3D stage: the tiles of many solves of one physics,
 // order and operand kind in one launch.  items[t] = {solve, first cell,
 // cells, 0}, the tiles of one solve consecutive; margs[solve] are the
-// solve's arguments of the stage launched (q_in / q_a / q_b / q_out, b,
+// solve's arguments of the stage launched (q_in / q_a / q_out, b,
 // c dt, mesh, boundaries, topology table).
 struct Tc3Batch {
   const Stage3DArgs<float>* margs;

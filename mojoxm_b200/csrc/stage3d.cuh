@@ -24,7 +24,7 @@
 //    tets' rows); only cube-boundary faces gather from global memory, with
 //    the neighbour cube and BC treatment of each cube face resolved once per
 //    tile.
-//  * q_a / q_b equal to q_in (SSPRK3 stages 1-3) are read from the tile, so
+//  * q_in, and q_a where it is q_in (SSPRK3 stage 1), are read from the tile, so
 //    each stage moves the algorithmic minimum of state bytes.
 //  * Where a tile's contraction works (element x RI-row group) would leave
 //    most of the block idle (FP32 P4 / P5), KS lanes of
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(NT, MINB) stage3d_kernel(Stage3DArgs<R> args, 
   uint32_t par = 0u;  // bit b: phase parity of tile buffer b
   int buf = 0;
   // the set-up above overlaps the previous stage's tail; its output (this
-  // stage's q_in / q_a / q_b, and q_out may be a buffer it still reads)
+  // stage's q_in / q_a, and q_out may be a buffer it still reads)
   // only after it has completed
   grid_dep_wait();
   if (tid == 0 && int(blockIdx.x) < ngroups && tile_bulk(blockIdx.x)) issue(blockIdx.x, 0);
@@ -283,8 +283,7 @@ __global__ void __launch_bounds__(NT, MINB) stage3d_kernel(Stage3DArgs<R> args, 
       }
     }
     __syncthreads();
-    // ---- contraction rhs = A B, source, RK combine (every stage's q_b is
-    // its q_in), floor, store
+    // ---- contraction rhs = A B, source, RK combine, floor, store
     const bool a_in = args.q_a == args.q_in;
     if constexpr (sizeof(R) == 8) {
       // FP64: a warp multiplies MG groups of 8 operator rows with 8 (element,

@@ -307,6 +307,8 @@ __global__ void __launch_bounds__(NT, MINB) stage3d_tc_kernel(Stage3DArgs<float>
     pend = 1u;
   }
   int buf = 0;
+  bool sourced = false;
+  if constexpr (Phys::kSource) sourced = ph.sourced();
   int cur_member = -1;  // batched: the solve whose arguments and table are loaded
   // ---- constant flux of each element of tile g (state tile qt), Fbar =
   // F(q at node 0), and its product with the four face normals: one thread
@@ -619,27 +621,42 @@ __global__ void __launch_bounds__(NT, MINB) stage3d_tc_kernel(Stage3DArgs<float>
       failed = true;
       break;
     }
-    if (warp < NT / 128 * 4) {  // warp w reads TMEM lanes [32 (w % 4), +32) (rows (c, slot)), columns
-       // [8 (w / 4), +8) of every 8 (NT / 128) and their lo halves, two such groups in flight
+    // warp w reads TMEM lanes [32 (w % 4), +32) (rows (c, slot)), of the
+    // operator rows the w / 4-th part, both halves of the accumulator; three
+    // groups of eight rows in flight (one for wide states, short of registers)
+    if (warp < NT / 128 * 4) {
       const int row = (warp & 3) * 32 + lane;
       const uint32_t lanes = tmem + (uint32_t((warp & 3) * 32) << 16);
-      constexpr int STEP = 8 * (NT / 128);
+      constexpr int U = NC <= 6 ? 3 : 1, WG = NT / 128, GROUPS = (S::NR / 8 + WG - 1) / WG;  // groups of eight rows a warp
+      const int first = WG == 1 ? 0 : (warp >> 2) * GROUPS;
 #pragma unroll
-      for (int c0 = (warp >> 2) * 8; c0 < S::NR; c0 += STEP) {
-        float v[8], w[8];
-        tmem_ld8(lanes + c0, v);
-        tmem_ld8(lanes + S::NR + c0, w);
+      for (int g0 = 0; g0 < GROUPS; g0 += U) {
+        float v[U][8], w[U][8];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          // (a group past the last reads the last again and stores nothing)
+          const int c0 = min((first + g0 + u) * 8, S::NR - 8);
+          if (g0 + u < GROUPS) {
+            tmem_ld8(lanes + c0, v[u]);
+            tmem_ld8(lanes + S::NR + c0, w[u]);
+          }
+        }
         tmem_ld_wait();
-        if (row < SL * NC)
+        if (row < SL * NC) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-          if (c0 + i < NP) sO[row * NPO + c0 + i] = v[i] + w[i];
+          for (int u = 0; u < U; ++u)
+            if (g0 + u < GROUPS) {
+              const int c0 = (first + g0 + u) * 8;
+#pragma unroll
+              for (int i = 0; i < 8; ++i)
+                if (c0 + i < NP) sO[row * NPO + c0 + i] = v[u][i] + w[u][i];
+            }
+        }
       }
     }
     tc_fence_before();
     __syncthreads();
-    // ---- epilogue per node: source, RK combine (every stage's q_b is its
-    // q_in), floor, store
+    // ---- epilogue per node: source, RK combine, floor, store
 #pragma unroll
     for (int r = 0; r < NEPI; ++r) {
       const int idx = tid + r * NT;
@@ -647,12 +664,16 @@ __global__ void __launch_bounds__(NT, MINB) stage3d_tc_kernel(Stage3DArgs<float>
         const int el = idx / NP, i = idx - el * NP, cl = el / 6, slot = (el - cl * 6) * EC + cl;
         const float* acc = sO + slot * NPO + i;
         const float* ql = TWO ? &q[idx * NC] : vq[TWO ? 0 : r];
-        float out[NC], src[NC];
-        if constexpr (Phys::kSource) ph.source(ql, src);
+        float out[NC];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          out[c] = acc[c * SL * NPO];
-          if constexpr (Phys::kSource) out[c] += src[c];
+        for (int c = 0; c < NC; ++c) out[c] = acc[c * SL * NPO];
+        if constexpr (Phys::kSource) {
+          if (sourced) {
+            float src[NC];
+            ph.source(ql, src);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) out[c] += src[c];
+          }
         }
         if (!args.rhs_only) {
 #pragma unroll
