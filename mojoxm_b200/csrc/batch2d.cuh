@@ -84,7 +84,7 @@ __device__ __forceinline__ void ssprk3_route(int stage, R* const* q, const R*& q
 }
 
 template <class R, class Phys, int NT>
-__global__ void __launch_bounds__(NT) stage2d_batch_kernel(Batch2DArgs<R> ba, Phys ph) {
+__global__ void __launch_bounds__(NT, Blocks2<R, Phys>::value) stage2d_batch_kernel(Batch2DArgs<R> ba, Phys ph) {
   constexpr int NC = Phys::NC;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);          // [2]

@@ -255,6 +255,7 @@ struct Stage2DArgs {
   R b, cdt;
   int nx, ny;
   int ncell;
+  int ec;  // cells per tile of a single solve's stage
   int bc[4];
   int rhs_only;
   int* err;

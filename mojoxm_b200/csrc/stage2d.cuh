@@ -3,7 +3,7 @@
 // Replaces the reference's two launches per stage -- *_face_flux_kernel_2d
 // (one thread per (face, slot) writing fstar to global memory) and
 // *_vol_lift_combine_rk_kernel_2d (src/local_mesh_2d_gpu_euler.mojo:33-144
-// and siblings) -- with one kernel.  A block owns EC whole cells (2
+// and siblings) -- with one kernel.  A block owns up to EC whole cells (2
 // triangles each, one contiguous span of q, bulk-copied into a
 // double-buffered shared tile), keeps one shared operator
 // A = [D_r | D_s | -Lift_0..2] for both triangle types (invJ applied to the
@@ -247,8 +247,28 @@ __device__ __forceinline__ void stage2d_tile(const Stage2DArgs<R>& args, const K
   }
 }
 
+// Blocks of 256 threads an SM holds: FP64 two (120 registers); FP32 the
+// physics whose flux takes more than 64 registers three (80, up to 100 B
+// spilled in the batched kernel), the others four.  The kernels are bound by
+// issue and latency, not by the tile's reuse: against two blocks with 100 KB
+// tiles the batched step of 64 limited HLLE solves takes 3.57 ms instead of
+// 3.93 where the tuned tiles leave room for three blocks, 3.76 instead of
+// 3.78 where one order's do not (four blocks of 64 registers: 3.92).
+template <class R, class Phys>
+struct Blocks2 {
+  static constexpr int value = sizeof(R) == 8 ? 2 : 4;
+};
+template <int F>
+struct Blocks2<float, Euler2D<float, F>> {
+  static constexpr int value = F == FLUX_RUSANOV ? 4 : 3;
+};
+template <bool GLM>
+struct Blocks2<float, Mhd2D<float, GLM>> {
+  static constexpr int value = 3;
+};
+
 template <class R, class Phys, int P, int EC, int NT>
-__global__ void __launch_bounds__(NT) stage2d_kernel(Stage2DArgs<R> args, KuhnTab2<R> tabp, Phys ph) {
+__global__ void __launch_bounds__(NT, Blocks2<R, Phys>::value) stage2d_kernel(Stage2DArgs<R> args, KuhnTab2<R> tabp, Phys ph) {
   constexpr int NC = Phys::NC;
   using S = Stage2DShape<P, NC, R>;
   constexpr int NP = S::NP, K = S::K, BSTR = S::BSTR;
@@ -263,7 +283,8 @@ __global__ void __launch_bounds__(NT) stage2d_kernel(Stage2DArgs<R> args, KuhnTa
   R* sA = sB + EB * BSTR;                                   // [K][NP]
   int2* sCd = reinterpret_cast<int2*>(sA + (K * NP + 1) / 2 * 2);  // [EC][4]
   const int tid = threadIdx.x;
-  const int ngroups = (args.ncell + EC - 1) / EC;
+  const int ec = args.ec;  // cells per tile, at most EC
+  const int ngroups = (args.ncell + ec - 1) / ec;
   if (tid == 0) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
@@ -277,7 +298,7 @@ __global__ void __launch_bounds__(NT) stage2d_kernel(Stage2DArgs<R> args, KuhnTa
   for (int idx = tid; idx < NP * K; idx += NT) sA[idx] = args.A[idx];
   __syncthreads();
   auto issue = [&](int grp, int buf) {
-    const int c0 = grp * EC, nc = min(EC, args.ncell - c0);
+    const int c0 = grp * ec, nc = min(ec, args.ncell - c0);
     const uint32_t bytes = uint32_t(nc) * 2u * NP * NC * sizeof(R);
     fence_proxy_async();
     mbar_arrive_expect_tx(&bar[buf], bytes);
@@ -291,8 +312,8 @@ __global__ void __launch_bounds__(NT) stage2d_kernel(Stage2DArgs<R> args, KuhnTa
   if (BULK && tid == 0 && int(blockIdx.x) < ngroups) issue(blockIdx.x, 0);
 
   for (int grp = blockIdx.x; grp < ngroups; grp += gridDim.x, buf ^= 1) {
-    const int cell0 = grp * EC;
-    const int ne_here = 2 * min(EC, args.ncell - cell0);
+    const int cell0 = grp * ec;
+    const int ne_here = 2 * min(ec, args.ncell - cell0);
     R* q = sQ + buf * QV;
     if (BULK) {
       if (!block_wait_bounded(&bar[buf], (par >> buf) & 1u, kWaitLimitNs2)) {
@@ -315,27 +336,71 @@ __global__ void __launch_bounds__(NT) stage2d_kernel(Stage2DArgs<R> args, KuhnTa
   }
 }
 
-template <class R, int P, int NC>
+template <class R, int P, class Phys>
 struct Cfg2 {
+  static constexpr int NC = Phys::NC;
   using S = Stage2DShape<P, NC, R>;
+  using Real = R;
   static constexpr int NP = S::NP;
   static constexpr size_t kFixed = 16 + (sizeof(KuhnTab2<R>) + 15) / 16 * 16 + sizeof(R) * (S::K * S::NP + 1);
-  static constexpr int EC_RAW = int((100 * 1024 - kFixed) / S::kPerCell);
-  static constexpr int EC = EC_RAW > 64 ? 64 : (EC_RAW < 1 ? 1 : EC_RAW);
+  // two, three or four blocks an SM, as the registers allow
+  static constexpr size_t kBudget = (sizeof(R) == 8 ? 100 : (Blocks2<R, Phys>::value == 3 ? 72 : 54)) * 1024;
+  static constexpr int EC_RAW = int((kBudget - kFixed) / S::kPerCell);
+  static constexpr int LN = sizeof(R) == 4 ? 2 : 1;  // cells per work item
+  static constexpr int EC = EC_RAW > 64 ? 64 : (EC_RAW < LN ? LN : EC_RAW / LN * LN);
   static constexpr int NT = 256;
   static constexpr size_t kSmem = kFixed + sizeof(R) * (2 * size_t(2 * EC) * S::NP * NC + size_t(2 * EC) * S::BSTR) + EC * 32;
 };
 
+// Cells per tile.  A large tile leaves SMs idle on a small mesh (64-cell
+// tiles of a 16^2 mesh: 4 blocks) and splits a larger one into uneven last
+// rounds; a small one leaves threads idle in every phase.  The rule takes the
+// size of least modelled time: the rounds of a block times the passes of its
+// three phases (latency: 16 units a pass, 4 a round), and an SM's share of
+// tiles times the warps their work items take (throughput: 1 unit a warp).
+// Tiles that do not end on 128 bytes split the stores' and loads' cache lines
+// between blocks: a fifth more.  Measured over 8^2..512^2, P = 1..5, every
+// size from 2 cells up (HLLE FP32 and FP64, shallow water FP32): the rule is
+// 0.8 % above the best size in the mean and 14 % at worst; always the largest
+// tile is 20 % and 80 %.  Times of a stage, largest tile of 100 KB -> now:
+// HLLE FP32 16^2 P3 12.4 -> 6.3 us, 100^2 P3 17.3 -> 12.0, 256^2 P3 62.4 ->
+// 54.4, 256^2 P5 129.7 -> 108.7; shallow water 256^2 P5 115 -> 84.
+template <class C>
+int tile_cells2(int ncell, int nsm, int bps) {
+  using S = typename C::S;
+  constexpr int G = S::NP / S::RI;
+  int64_t best = INT64_MAX;
+  int ec = C::EC;
+  for (int e = C::EC; e > 0; e -= C::LN) {
+    const int tiles = (ncell + e - 1) / e, rounds = (tiles + nsm * bps - 1) / (nsm * bps), per_sm = (tiles + nsm - 1) / nsm;
+    const int items[3] = {e / C::LN * 2 * S::NP, e / C::LN * 5 * S::NFP, 2 * e * G};
+    int64_t passes = 0, warps = 0;
+    for (int n : items) {
+      passes += (n + C::NT - 1) / C::NT;
+      warps += (n + 31) / 32;
+    }
+    int64_t cost = rounds * (16 * passes + 4) + per_sm * warps;
+    if (size_t(e) * 2 * S::NP * C::NC * sizeof(typename C::Real) % 128 != 0) cost += cost / 5;
+    if (cost < best) {
+      best = cost;
+      ec = e;
+    }
+  }
+  return ec;
+}
+
 template <class R, class Phys, int P>
-cudaError_t launch2_p(const Stage2DArgs<R>& a, const KuhnTab2<R>& tab, const Phys& ph, int nsm, cudaStream_t st) {
-  using C = Cfg2<R, P, Phys::NC>;
+cudaError_t launch2_p(const Stage2DArgs<R>& args, const KuhnTab2<R>& tab, const Phys& ph, int nsm, cudaStream_t st) {
+  using C = Cfg2<R, P, Phys>;
   auto kern = stage2d_kernel<R, Phys, P, C::EC, C::NT>;
   static int bps = -1;
   if (bps < 0) {
     cudaError_t e = persistent_blocks_per_sm((const void*)kern, C::NT, C::kSmem, &bps);
     if (e != cudaSuccess) return e;
   }
-  const int ngroups = (a.ncell + C::EC - 1) / C::EC;
+  Stage2DArgs<R> a = args;
+  a.ec = tile_cells2<C>(a.ncell, nsm, bps);
+  const int ngroups = (a.ncell + a.ec - 1) / a.ec;
   int nblk = nsm * bps;
   if (nblk > ngroups) nblk = ngroups;
   if (nblk < 1) nblk = 1;

@@ -1,8 +1,10 @@
 """The 2D stage at the edges of its tiles, and the limiter at the edges of its
 chunks.
 
-The 2D stage takes cells in pairs (FP32) inside tiles of up to 64 cells;
-odd cell counts leave a pair with one cell, 65 and 129 cells a tile of one.
+The 2D stage takes cells in pairs (FP32) inside tiles of 2 to 64 cells, the
+size by mesh and order; odd cell counts leave a pair with one cell, and meshes
+of 65 to 20,000 cells take small tiles, one round of larger ones and several
+rounds, with partial last tiles.
 The limiter works in chunks of 128 elements: meshes on both sides of one and
 two chunks, with every boundary kind.  Right-hand sides and limited states are
 compared with the FP64 oracle; bounds: FP32 arithmetic over K <= 60 columns of
@@ -34,6 +36,22 @@ def test_rhs_on_partial_tiles_2d(oracle_mod, name, P, prec, bcs):
         err = C.rel_err(s.rhs(q), o.rhs(q))
         s.close()
         assert err < (4e-6 if prec == "f32" else C.TOL_F64_2D[P]), (n, err)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("name,P", [("euler_hlle", 1), ("euler_hlle", 3), ("euler_rusanov", 5), ("shallow_water", 4),
+                                    ("mhd_glm", 2)])
+@pytest.mark.parametrize("n", [(61, 59), (150, 131)])
+def test_rhs_on_many_tiles_2d(oracle_mod, name, P, prec, n):
+    ph, L = C.PHYSICS_2D[name](), (1.0, 0.8)
+    s = M.Solver(M.Mesh(*n, 1, *L, 1.0, bcs=M.BoundaryConditions(*C.BCS_2D["inflow_outflow"], 0, 0), dim=2), ph, P=P,
+                 precision=prec)
+    o = oracle_mod.Oracle2D(P, n, L, M.physics_dict(ph), C.BCS_2D["inflow_outflow"])
+    q = C.random_state(s.shape, ph, seed=sum(n)).astype(np.float32).astype(np.float64)
+    err = C.rel_err(s.rhs(q), o.rhs(q))
+    s.close()
+    assert err < (4e-6 if prec == "f32" else C.TOL_F64_2D[P]), (n, err)
 
 
 @pytest.mark.gpu
