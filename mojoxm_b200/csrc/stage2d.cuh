@@ -252,8 +252,8 @@ __device__ __forceinline__ void stage2d_tile(const Stage2DArgs<R>& args, const K
 // spilled in the batched kernel), the others four.  The kernels are bound by
 // issue and latency, not by the tile's reuse: against two blocks with 100 KB
 // tiles the batched step of 64 limited HLLE solves takes 3.57 ms instead of
-// 3.93 where the tuned tiles leave room for three blocks, 3.76 instead of
-// 3.78 where one order's do not (four blocks of 64 registers: 3.92).
+// 3.93 in a row of ten steps, 3.76 instead of 3.78 in passes of their own
+// (four blocks of 64 registers: 3.92 in a row).
 template <class R, class Phys>
 struct Blocks2 {
   static constexpr int value = sizeof(R) == 8 ? 2 : 4;
